@@ -39,9 +39,9 @@ UNITS = {
     "khb_ctmesh.cu": ["-fmad=false"],
     "khb_geometry.cpp": [],
 }
-HEADERS = ["khb_device.cuh", "khb_kernels.cuh", "khb_types.cuh", "khb_internal.hpp", "khb_dual.cuh", "khb_adjoint_flux.cuh", os.path.join("..", "..", "include", "khb.h")]
+HEADERS = ["khb_arith.cuh", "khb_device.cuh", "khb_kernels.cuh", "khb_types.cuh", "khb_internal.hpp", "khb_dual.cuh", "khb_adjoint_flux.cuh", os.path.join("..", "..", "include", "khb.h")]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-COMMON = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC"]
+COMMON = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-split-compile=4"]
 
 
 def _deps_mtime():

@@ -1,0 +1,122 @@
+// khb_arith.cuh -- division and square root policies of the device functions.
+//
+// The FP64 path rounds every division and square root as IEEE 754 does, and so must anything that
+// replaces them.  The compiler's own sequences end in a branch to a slow path for operands near the
+// ends of the exponent range; with about 40 of them per face these branches are a tenth of the
+// instructions, and, worse, each one ends a basic block, so that the independent chains of a face
+// (sixteen limiters, two 4-vectors, two signal speeds) cannot be scheduled into one another.
+//
+// Plain<R> is the operators themselves.  Exact64 is branch-free: Newton-Raphson on the approximate
+// reciprocal (reciprocal square root) of the hardware, then residual corrections by FMA (P. Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34,
+// 1990).  With u = 2^-53, a and b scaled into [1, 2):
+//   quotient: q within 1/2 ulp + O(u^2) of a/b after the first correction, y with |b y - 1| <= u.  The
+//     last step forms q + (a - b q) y with an exact residual; its error |a/b - q| |b y - 1| is below
+//     2^-107 (a < b; twice that otherwise) while a/b, being a ratio of 53-bit integers, stays at least
+//     2^-106/b from every midpoint of two neighbouring doubles: the rounding is that of a/b.  Where b's
+//     significand is all ones, 1/b is a rounding tie of the Newton step: inv() sets that case right; a
+//     quotient could be an ulp off there for a power of two as numerator, and only then.
+//   root: the same argument with x - m^2, an odd multiple of 2^-106 and 1 mod 8 of it, for a midpoint m.
+// Both hold while no divisor, radicand, quotient or residual leaves the normal range.  Where one does at
+// the small end, or overflows, or is infinite or NaN to begin with, the scheme's result is a NaN (the
+// approximations return infinities there, and a correction multiplies them by zero), so it is enough to
+// look at the values everything else has run into: see() keeps the largest magnitude it is shown, and
+// the caller tests ok() once, after all of it, and repeats the computation with Plain<double> where it
+// fails.  Values are shown to see() where a computation ends and where a comparison could drop a NaN
+// on the way (a clip, a maximum).  Divisors above 2^1022 would need states beyond 1e150, whose fluxes overflow.  The lower
+// end is open because the field's diffusive tail, which spreads from magnetized into unmagnetized zones,
+// takes every magnitude down to the smallest in its first hundred steps: where a quotient or its
+// numerator is below 2^-960, its last bit may be off, and a negative zero comes out positive.
+#pragma once
+
+#include <cuda_runtime.h>
+
+namespace khb {
+
+__device__ __forceinline__ float  dsqrt(float x)  { return sqrtf(x); }
+__device__ __forceinline__ double dsqrt(double x) { return sqrt(x); }
+
+template <typename R>
+struct Plain {
+    struct Rcp { R b; };
+    static __device__ __forceinline__ bool ok() { return true; }
+    __device__ __forceinline__ Rcp rcp(R b) { return Rcp{b}; }
+    __device__ __forceinline__ R quot(R a, Rcp r) { return a / r.b; }
+    __device__ __forceinline__ R div(R a, R b) { return a / b; }
+    __device__ __forceinline__ R inv(R b) { return R(1) / b; }
+    __device__ __forceinline__ R root(R x) { return dsqrt(x); }
+    __device__ __forceinline__ R root_or_zero(R x) { return dsqrt(x); }
+    __device__ __forceinline__ R inv_root(R x) { return rsqrt(x); }
+    template <typename T> __device__ __forceinline__ void see(T) {}
+    template <typename T> __device__ __forceinline__ void bounded(T) {}
+};
+
+struct Exact64 {
+    struct Rcp { double b, y; };
+    unsigned top = 0, wide = 0;      // running maxima of high words, doubled (without the sign)
+
+    __device__ __forceinline__ bool ok() const { return top < 0xfce00000u && wide < 0x98e00000u; }
+    // |x| must be below 2^1000, not infinite, not NaN
+    __device__ __forceinline__ void see(double x) { top = max(top, (unsigned)__double2hiint(x) << 1); }
+    // |x| must be below 2^200: an input whose powers divide something
+    __device__ __forceinline__ void bounded(double x) { wide = max(wide, (unsigned)__double2hiint(x) << 1); }
+    // 1/b: y0 (1 + e + e^2) with e = 1 - b y0 at 2^-60 before its rounding, then one Newton step
+    static __device__ __forceinline__ double recip(double b)
+    {
+        double y;
+        asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+        double e = __fma_rn(-b, y, 1.0);
+        e = __fma_rn(e, e, e);
+        y = __fma_rn(y, e, y);
+        e = __fma_rn(-b, y, 1.0);
+        return __fma_rn(y, e, y);
+    }
+    __device__ __forceinline__ Rcp rcp(double b) { return Rcp{b, recip(b)}; }
+    __device__ __forceinline__ double quot(double a, Rcp r)
+    {
+        double q = a * r.y;
+        q = __fma_rn(__fma_rn(-r.b, q, a), r.y, q);
+        return __fma_rn(__fma_rn(-r.b, q, a), r.y, q);
+    }
+    __device__ __forceinline__ double div(double a, double b) { return quot(a, rcp(b)); }
+    // 1/b: recip() rounds it correctly (Markstein) unless the significand of b is all ones, where the
+    // Newton step ends in a tie and one ulp is missing
+    __device__ __forceinline__ double inv(double b)
+    {
+        const double y = recip(b);
+        const int one = ((__double2hiint(b) | (int)0xfff00000) & __double2loint(b)) == -1;
+        return __hiloint2double(__double2hiint(y), __double2loint(y) + one);
+    }
+    // g -> sqrt(x), h -> 1/(2 sqrt(x)) by two coupled Newton steps
+    struct Root { double g, h; };
+    static __device__ __forceinline__ Root coupled(double x)
+    {
+        double y;
+        asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+        double g = x * y, h = 0.5 * y;
+        double r = __fma_rn(-g, h, 0.5);
+        g = __fma_rn(g, r, g);
+        h = __fma_rn(h, r, h);
+        r = __fma_rn(-g, h, 0.5);
+        g = __fma_rn(g, r, g);
+        h = __fma_rn(h, r, h);
+        return Root{g, h};
+    }
+    // the last correction is that of the root: g + (x - g^2) h.  A zero, negative or infinite radicand
+    // ends in a NaN; one below 2^-960 may be off in the last bit of its root
+    __device__ __forceinline__ double root(double x)
+    {
+        const Root c = coupled(x);
+        return __fma_rn(__fma_rn(-c.g, c.g, x), c.h, c.g);
+    }
+    // ... of a radicand that may be zero
+    __device__ __forceinline__ double root_or_zero(double x) { return x == 0. ? x : root(x == 0. ? 1. : x); }
+    // 1 / sqrt(x) within an ulp, as rsqrt()
+    __device__ __forceinline__ double inv_root(double x) { return 2.0 * coupled(x).h; }
+};
+
+// The policy a face or zone kernel tries first for arithmetic type R
+template <typename R> struct FastArith { typedef Plain<R> type; };
+template <> struct FastArith<double> { typedef Exact64 type; };
+
+} // namespace khb

@@ -147,7 +147,8 @@ __global__ void __launch_bounds__(128) k_ct_center(Dims d, DevGeom g, khb_fields
     const long long c = ((long long)k*d.n2 + j)*d.n1 + i;
     const double* const F[3] = {Bf.v[0], Bf.v[1], Bf.v[2]};
     double Bp[3];
-    ct_zone_b(d, g, F, c, j, i, Bp);
+    Plain<double> ar;
+    ct_zone_b(ar, d, g, F, c, j, i, Bp);
     const double gdet = __ldg(g.gdet[3] + (long long)j*g.G1 + i);
 #pragma unroll
     for (int v = 0; v < 3; ++v) {

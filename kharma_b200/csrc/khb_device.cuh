@@ -10,6 +10,7 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "khb_arith.cuh"
 #include "khb_types.cuh"
 
 namespace khb {
@@ -19,8 +20,6 @@ template <typename R> __device__ __forceinline__ R kmax(R a, R b) { return (a < 
 template <typename R> __device__ __forceinline__ R kmin(R a, R b) { return (b < a) ? b : a; }
 template <typename R> __device__ __forceinline__ R kclip(R n, R lo, R hi) { return kmin(kmax(lo, n), hi); }
 
-__device__ __forceinline__ float  dsqrt(float x)  { return sqrtf(x); }
-__device__ __forceinline__ double dsqrt(double x) { return sqrt(x); }
 __device__ __forceinline__ float  dabs(float x)   { return fabsf(x); }
 __device__ __forceinline__ double dabs(double x)  { return fabs(x); }
 
@@ -35,6 +34,15 @@ enum { EX_LINEAR_VL = 1, EX_WENO5_LINEAR = 2, EX_PPMX = 3, EX_MP5 = 4 };
 
 // ------------------------------------------------------------------ reconstruction
 // flux/reconstruction.hpp:52-56
+template <typename R, class AR>
+__device__ __forceinline__ R mc_lim(AR& ar, R dm, R dp)
+{
+    const bool nz = dabs(dp) > R(0);
+    const R q = ar.div(dm, nz ? dp : R(1));
+    const R r = nz ? q : R(2);
+    // the reference's max(0, min(2, min(2 r, (1 + r)/2))), its operands in the order that keeps a NaN
+    return kmax(kmin(kmin(R(2)*r, R(0.5)*(R(1)+r)), R(2)), R(0));
+}
 template <typename R>
 __device__ __forceinline__ R mc_lim(R dm, R dp)
 {
@@ -42,14 +50,20 @@ __device__ __forceinline__ R mc_lim(R dm, R dp)
     return kmax(R(0), kmin(R(2), kmin(R(2)*r, R(0.5)*(R(1)+r))));
 }
 
+// WENO5 weights are FP64 in both forms: the face's policy where it is one for FP64, else the operators.
+// With inputs below 2^200 (the face checks them) the denominators lie in [1e-52, 2^830] and the weights
+// in [2^-830, 2^170]: no division of the weights leaves the normal range.
+__device__ __forceinline__ Exact64& weights_of(Exact64& ar) { return ar; }
+template <typename R> __device__ __forceinline__ Plain<double> weights_of(Plain<R>&) { return Plain<double>(); }
+
 // Value at the right face of a zone with stencil x1..x5 (reconstruct_right, :114-204, :351-394)
-template <int RECON, typename R>
-__device__ __forceinline__ R recon_right(R x1, R x2, R x3, R x4, R x5)
+template <int RECON, typename R, class AR>
+__device__ __forceinline__ R recon_right(AR& ar, R x1, R x2, R x3, R x4, R x5)
 {
     if (RECON == RECON_DONOR) {
         return x3;
     } else if (RECON == RECON_MC) {
-        return x3 + R(0.5)*(mc_lim(x3 - x2, x4 - x3)*(x4 - x3));
+        return x3 + R(0.5)*(mc_lim(ar, x3 - x2, x4 - x3)*(x4 - x3));
     } else if (RECON == RECON_WENO5) {
         // WENO5-JS (T07 A18, S11 8-9), reconstruction.hpp:183-204.  Weights are always formed in
         // FP64: with EPS = 1e-26 the squared denominators underflow FP32.
@@ -63,15 +77,16 @@ __device__ __forceinline__ R recon_right(R x1, R x2, R x3, R x4, R x5)
         b2 = (13./12.)*c1*c1 + (1./4.)*c2*c2;
         double d0 = 1.e-26 + b0, d1 = 1.e-26 + b1, d2 = 1.e-26 + b2;
         d0 *= d0; d1 *= d1; d2 *= d2;
-        const double w0 = (1./16.)/d0, w1 = (5./8.)/d1, w2 = (5./16.)/d2;
-        const double W = w0 + w1 + w2;
-        return (R)(((3./8.)*y1 - (5./4.)*y2 + (15./8.)*y3)*(w0 / W) +
-                   ((-1./8.)*y2 + (3./4.)*y3 + (3./8.)*y4)*(w1 / W) +
-                   ((3./8.)*y3 + (3./4.)*y4 - (1./8.)*y5)*(w2 / W));
+        auto&& wr = weights_of(ar);
+        const double w0 = wr.quot(1./16., wr.rcp(d0)), w1 = wr.quot(5./8., wr.rcp(d1)), w2 = wr.quot(5./16., wr.rcp(d2));
+        const auto W = wr.rcp(w0 + w1 + w2);
+        return (R)(((3./8.)*y1 - (5./4.)*y2 + (15./8.)*y3)*wr.quot(w0, W) +
+                   ((-1./8.)*y2 + (3./4.)*y3 + (3./8.)*y4)*wr.quot(w1, W) +
+                   ((3./8.)*y3 + (3./4.)*y4 - (1./8.)*y5)*wr.quot(w2, W));
     } else {
         // PPM (Colella & Woodward with CS limiters), reconstruction.hpp:351-381: qrv
-        R qlv = (R(7)*(x3 + x2) - (x1 + x4))/R(12);
-        R qrv = (R(7)*(x3 + x4) - (x2 + x5))/R(12);
+        R qlv = ar.div(R(7)*(x3 + x2) - (x1 + x4), R(12));
+        R qrv = ar.div(R(7)*(x3 + x4) - (x2 + x5), R(12));
         qlv = kmax(qlv, kmin(x3, x2));
         qlv = kmin(qlv, kmax(x3, x2));
         qrv = kmax(qrv, kmin(x3, x4));
@@ -83,13 +98,13 @@ __device__ __forceinline__ R recon_right(R x1, R x2, R x3, R x4, R x5)
     }
 }
 // Value at the left face of a zone (reconstruct_left, :114-204, :351-394)
-template <int RECON, typename R>
-__device__ __forceinline__ R recon_left(R x1, R x2, R x3, R x4, R x5)
+template <int RECON, typename R, class AR>
+__device__ __forceinline__ R recon_left(AR& ar, R x1, R x2, R x3, R x4, R x5)
 {
     if (RECON == RECON_DONOR) {
         return x3;
     } else if (RECON == RECON_MC) {
-        return x3 - R(0.5)*(mc_lim(x3 - x2, x4 - x3)*(x4 - x3));
+        return x3 - R(0.5)*(mc_lim(ar, x3 - x2, x4 - x3)*(x4 - x3));
     } else if (RECON == RECON_WENO5) {
         const double y1 = x1, y2 = x2, y3 = x3, y4 = x4, y5 = x5;
         double c1, c2, b0, b1, b2;
@@ -101,14 +116,15 @@ __device__ __forceinline__ R recon_left(R x1, R x2, R x3, R x4, R x5)
         b2 = (13./12.)*c1*c1 + (1./4.)*c2*c2;
         double d0 = 1.e-26 + b0, d1 = 1.e-26 + b1, d2 = 1.e-26 + b2;
         d0 *= d0; d1 *= d1; d2 *= d2;
-        const double w0 = (1./16.)/d2, w1 = (5./8.)/d1, w2 = (5./16.)/d0;
-        const double W = w0 + w1 + w2;
-        return (R)(((3./8.)*y5 - (5./4.)*y4 + (15./8.)*y3)*(w0 / W) +
-                   ((-1./8.)*y4 + (3./4.)*y3 + (3./8.)*y2)*(w1 / W) +
-                   ((3./8.)*y3 + (3./4.)*y2 - (1./8.)*y1)*(w2 / W));
+        auto&& wr = weights_of(ar);
+        const double w0 = wr.quot(1./16., wr.rcp(d2)), w1 = wr.quot(5./8., wr.rcp(d1)), w2 = wr.quot(5./16., wr.rcp(d0));
+        const auto W = wr.rcp(w0 + w1 + w2);
+        return (R)(((3./8.)*y5 - (5./4.)*y4 + (15./8.)*y3)*wr.quot(w0, W) +
+                   ((-1./8.)*y4 + (3./4.)*y3 + (3./8.)*y2)*wr.quot(w1, W) +
+                   ((3./8.)*y3 + (3./4.)*y2 - (1./8.)*y1)*wr.quot(w2, W));
     } else {
-        R qlv = (R(7)*(x3 + x2) - (x1 + x4))/R(12);
-        R qrv = (R(7)*(x3 + x4) - (x2 + x5))/R(12);
+        R qlv = ar.div(R(7)*(x3 + x2) - (x1 + x4), R(12));
+        R qrv = ar.div(R(7)*(x3 + x4) - (x2 + x5), R(12));
         qlv = kmax(qlv, kmin(x3, x2));
         qlv = kmin(qlv, kmax(x3, x2));
         qrv = kmax(qrv, kmin(x3, x4));
@@ -118,6 +134,19 @@ __device__ __forceinline__ R recon_left(R x1, R x2, R x3, R x4, R x5)
         if (dabs(qd) >= R(2)*dabs(qc)) qlv = x3 - R(2)*qc;
         return qlv;
     }
+}
+
+template <int RECON, typename R>
+__device__ __forceinline__ R recon_right(R x1, R x2, R x3, R x4, R x5)
+{
+    Plain<R> ar;
+    return recon_right<RECON, R>(ar, x1, x2, x3, x4, x5);
+}
+template <int RECON, typename R>
+__device__ __forceinline__ R recon_left(R x1, R x2, R x3, R x4, R x5)
+{
+    Plain<R> ar;
+    return recon_left<RECON, R>(ar, x1, x2, x3, x4, x5);
 }
 
 // ------------------------------------------------------------------ further reconstructions
@@ -315,20 +344,22 @@ __device__ __forceinline__ void lower4(const R g[4][4], const R* vcon, R* vcov)
 
 // grmhd_functions.hpp:121-133
 template <typename R>
-__device__ __forceinline__ R lorentz(const R g[4][4], R u1, R u2, R u3)
+__device__ __forceinline__ R lorentz_sq(const R g[4][4], R u1, R u2, R u3)
 {
     const R qsq = g[1][1] * u1 * u1 + g[2][2] * u2 * u2 + g[3][3] * u3 * u3 +
                   R(2.) * (g[1][2] * u1 * u2 + g[1][3] * u1 * u3 + g[2][3] * u2 * u3);
-    return dsqrt(R(1.) + qsq);
+    return R(1.) + qsq;
 }
+template <typename R>
+__device__ __forceinline__ R lorentz(const R g[4][4], R u1, R u2, R u3) { return dsqrt(lorentz_sq(g, u1, u2, u3)); }
 
 // grmhd_functions.hpp:225-246.  P = {rho, u, u1, u2, u3, B1, B2, B3}
-template <typename R, bool HAS_B>
-__device__ __forceinline__ void calc_4vecs(const R g[4][4], R gcon00, const R* gcon0, const R* P, FourVec<R>& D)
+template <typename R, bool HAS_B, class AR>
+__device__ __forceinline__ void calc_4vecs(AR& ar, const R g[4][4], R gcon00, const R* gcon0, const R* P, FourVec<R>& D)
 {
-    const R gamma = lorentz(g, P[2], P[3], P[4]);
-    const R alpha = R(1.) / dsqrt(-gcon00);
-    D.ucon[0] = gamma / alpha;
+    const R gamma = ar.root(lorentz_sq(g, P[2], P[3], P[4]));
+    const R alpha = ar.inv(ar.root(-gcon00));
+    D.ucon[0] = ar.div(gamma, alpha);
 #pragma unroll
     for (int v = 0; v < 3; ++v) D.ucon[v+1] = P[2 + v] - gamma * alpha * gcon0[v+1];
     lower4(g, D.ucon, D.ucov);
@@ -337,13 +368,21 @@ __device__ __forceinline__ void calc_4vecs(const R g[4][4], R gcon00, const R* g
 #pragma unroll
         for (int v = 0; v < 3; ++v) b0 += P[5 + v] * D.ucov[v+1];
         D.bcon[0] = b0;
+        const auto ru0 = ar.rcp(D.ucon[0]);
 #pragma unroll
-        for (int v = 0; v < 3; ++v) D.bcon[v+1] = (P[5 + v] + b0 * D.ucon[v+1]) / D.ucon[0];
+        for (int v = 0; v < 3; ++v) D.bcon[v+1] = ar.quot(P[5 + v] + b0 * D.ucon[v+1], ru0);
         lower4(g, D.bcon, D.bcov);
     } else {
 #pragma unroll
         for (int mu = 0; mu < 4; ++mu) D.bcon[mu] = D.bcov[mu] = R(0);
     }
+}
+
+template <typename R, bool HAS_B>
+__device__ __forceinline__ void calc_4vecs(const R g[4][4], R gcon00, const R* gcon0, const R* P, FourVec<R>& D)
+{
+    Plain<R> ar;
+    calc_4vecs<R, HAS_B>(ar, g, gcon00, gcon0, P, D);
 }
 
 // One row T^dir_mu of the MHD (or hydro) stress tensor, grmhd_functions.hpp:51-60, 142-155
@@ -389,8 +428,8 @@ __device__ __forceinline__ void prim_to_flux(const R* P, const FourVec<R>& D, R 
 }
 
 // The fast-magnetosonic signal speeds along dir for a given cms2 (flux_functions.hpp:411-438)
-template <typename R>
-__device__ __forceinline__ void vchar_speeds(R cms2, const FourVec<R>& D, R gcon00, R gcon0d, R gcondd, int dir,
+template <typename R, class AR>
+__device__ __forceinline__ void vchar_speeds(AR& ar, R cms2, const FourVec<R>& D, R gcon00, R gcon0d, R gcondd, int dir,
                                              R& cmax, R& cmin)
 {
     const R Asq = gcondd, Bsq = gcon00, AB = gcon0d;
@@ -398,79 +437,98 @@ __device__ __forceinline__ void vchar_speeds(R cms2, const FourVec<R>& D, R gcon
     const R A  = Bu*Bu - (Bsq + Bu*Bu) * cms2;
     const R Bq = R(2.) * (Au*Bu - (AB + Au*Bu) * cms2);
     const R Cq = Au*Au - (Asq + Au*Au) * cms2;
-    const R discr = dsqrt(kmax(Bq * Bq - R(4.) * A * Cq, R(0)));
-    const R vp = -(-Bq + discr) / (R(2.) * A);
-    const R vm = -(-Bq - discr) / (R(2.) * A);
+    const R discr = ar.root(kmax(Bq * Bq - R(4.) * A * Cq, R(0)));
+    const auto r2A = ar.rcp(R(2.) * A);
+    const R vp = ar.quot(-(-Bq + discr), r2A);
+    const R vm = ar.quot(-(-Bq - discr), r2A);
+    ar.see(vp);
+    ar.see(vm);
     cmax = kmax(vp, vm);
     cmin = kmin(vp, vm);
+}
+template <typename R>
+__device__ __forceinline__ void vchar_speeds(R cms2, const FourVec<R>& D, R gcon00, R gcon0d, R gcondd, int dir,
+                                             R& cmax, R& cmin)
+{
+    Plain<R> ar;
+    vchar_speeds<R>(ar, cms2, D, gcon00, gcon0d, gcondd, dir, cmax, cmin);
 }
 
 // flux_functions.hpp:368-439.  The reference discards its clip() results (:378, :409), so no
 // clipping happens here either.  With A_mu = delta^dir_mu and B_mu = delta^0_mu the raised
 // vectors and their contractions reduce exactly to single metric entries.
-template <typename R, bool HAS_B>
-__device__ __forceinline__ void vchar(const R* P, const FourVec<R>& D, R gam, R gcon00, R gcon0d, R gcondd,
+template <typename R, bool HAS_B, class AR>
+__device__ __forceinline__ void vchar(AR& ar, const R* P, const FourVec<R>& D, R gam, R gcon00, R gcon0d, R gcondd,
                                       int dir, R& cmax, R& cmin)
 {
     const R ef  = P[0] + gam * P[1];
-    const R cs2 = gam * (gam - R(1)) * P[1] / ef;
+    const R cs2 = ar.div(gam * (gam - R(1)) * P[1], ef);
     R cms2;
     if (HAS_B) {
         const R bsq = dot4(D.bcon, D.bcov);
-        const R va2 = bsq / (bsq + ef);
+        const R va2 = ar.div(bsq, bsq + ef);
         cms2 = cs2 + va2 - cs2 * va2;
     } else {
         cms2 = cs2;
     }
-    vchar_speeds<R>(cms2, D, gcon00, gcon0d, gcondd, dir, cmax, cmin);
+    vchar_speeds<R>(ar, cms2, D, gcon00, gcon0d, gcondd, dir, cmax, cmin);
+}
+template <typename R, bool HAS_B>
+__device__ __forceinline__ void vchar(const R* P, const FourVec<R>& D, R gam, R gcon00, R gcon0d, R gcondd,
+                                      int dir, R& cmax, R& cmin)
+{
+    Plain<R> ar;
+    vchar<R, HAS_B>(ar, P, D, gam, gcon00, gcon0d, gcondd, dir, cmax, cmin);
 }
 
 // ------------------------------------------------------------------ 1D_W inversion (FP64)
 enum Status { ST_SUCCESS = 0, ST_NEG_INPUT, ST_MAX_ITER, ST_BAD_UT, ST_BAD_GAMMA, ST_NEG_RHO, ST_NEG_U, ST_NEG_RHOU };
 
 // onedw.hpp:49-67
-__device__ __forceinline__ double lorentz_calc_w(double Bsq, double D, double QdB, double Qtsq, double Wp)
+template <class AR>
+__device__ __forceinline__ double lorentz_calc_w(AR& ar, double Bsq, double D, double QdB, double Qtsq, double Wp)
 {
     const double QdBsq = QdB * QdB;
     const double W = Wp + D;
     const double W2 = W * W;
     const double WB = W + Bsq;
-    const double utsq = -((W + WB) * QdBsq + W2 * Qtsq) / (QdBsq * (W + WB) + W2 * (Qtsq - WB * WB));
-    if (utsq < -1.e-15 || utsq > 1.e7) return -1.;
-    return sqrt(1. + fabs(utsq));
+    const double utsq = ar.div(-((W + WB) * QdBsq + W2 * Qtsq), QdBsq * (W + WB) + W2 * (Qtsq - WB * WB));
+    const double gamma = ar.root(1. + fabs(utsq));
+    return (utsq < -1.e-15 || utsq > 1.e7) ? -1. : gamma;
 }
 // onedw.hpp:72-84
-__device__ __forceinline__ double err_eqn(double gam, double Bsq, double D, double Ep, double QdB, double Qtsq,
+template <class AR>
+__device__ __forceinline__ double err_eqn(AR& ar, double gam, double Bsq, double D, double Ep, double QdB, double Qtsq,
                                           double Wp, int& eflag)
 {
     const double W = Wp + D;
-    const double gamma = lorentz_calc_w(Bsq, D, QdB, Qtsq, Wp);
+    const double gamma = lorentz_calc_w(ar, Bsq, D, QdB, Qtsq, Wp);
     if (gamma < 1) eflag = ST_BAD_UT;
-    const double w = W / (gamma*gamma);
-    const double rho = D / gamma;
-    const double p = (w - rho) * (gam - 1) / gam;
-    return -Ep + Wp - p + 0.5 * Bsq + 0.5 * (Bsq * Qtsq - QdB * QdB) / ((Bsq + W)*(Bsq + W));
+    const double w = ar.div(W, gamma*gamma);
+    const double rho = ar.div(D, gamma);
+    const double p = ar.div((w - rho) * (gam - 1), gam);
+    return -Ep + Wp - p + 0.5 * Bsq + ar.div(0.5 * (Bsq * Qtsq - QdB * QdB), (Bsq + W)*(Bsq + W));
 }
 
 // The same residual with one division and one reciprocal square root in place of four divisions
 // and a square root: 1/gamma = rsqrt(1 + |utsq|), rho = D/gamma and w = W/gamma^2 by products,
 // (gam-1)/gam from the caller (gfac), (Bsq + W)^2 = WB^2.  Equal to err_eqn up to rounding (a few
 // ulp); used by the FP32-flux form's inversion, which has no bitwise contract with the reference.
-__device__ __forceinline__ double err_eqn_fast(double gfac, double Bsq, double D, double Ep, double QdB, double Qtsq,
+template <class AR>
+__device__ __forceinline__ double err_eqn_fast(AR& ar, double gfac, double Bsq, double D, double Ep, double QdB, double Qtsq,
                                                double Wp, int& eflag)
 {
     const double QdBsq = QdB * QdB;
     const double W = Wp + D;
     const double W2 = W * W;
     const double WB = W + Bsq;
-    const double utsq = -((W + WB) * QdBsq + W2 * Qtsq) / (QdBsq * (W + WB) + W2 * (Qtsq - WB * WB));
-    double ig;                                   // 1/gamma; gamma = -1 for an unphysical utsq
+    const double utsq = ar.div(-((W + WB) * QdBsq + W2 * Qtsq), QdBsq * (W + WB) + W2 * (Qtsq - WB * WB));
+    double ig = ar.inv_root(1. + fabs(utsq));    // 1/gamma; gamma = -1 for an unphysical utsq
     if (utsq < -1.e-15 || utsq > 1.e7) { ig = -1.; eflag = ST_BAD_UT; }
-    else ig = rsqrt(1. + fabs(utsq));
     const double w = W * (ig * ig);
     const double rho = D * ig;
     const double p = (w - rho) * gfac;
-    return -Ep + Wp - p + 0.5 * Bsq + 0.5 * (Bsq * Qtsq - QdBsq) / (WB * WB);
+    return -Ep + Wp - p + 0.5 * Bsq + ar.div(0.5 * (Bsq * Qtsq - QdBsq), WB * WB);
 }
 
 // Zone-centre geometry for the inversion, floors and P->U
@@ -491,17 +549,29 @@ __device__ __forceinline__ void raise4(const ZoneGeom& G, const double* vcov, do
     }
 }
 
+// |a / b| < tol as the rounded quotient compares, without the division unless the product is within
+// a few ulp of deciding (the rounding errors of tol |b| and of the quotient are below 2^-52 together)
+__device__ __forceinline__ bool ratio_below(double a, double b, double tol)
+{
+    const double x = fabs(a), y = tol * fabs(b);
+    if (y > 1e-290 && y < 1e290) {
+        if (x < y * (1. - 1e-14)) return true;
+        if (x > y * (1. + 1e-14)) return false;
+    }
+    return fabs(a / b) < tol;
+}
+
 // onedw.hpp:89-233.  U: conserved zone values; P: guess on entry, updated only on success.
 // The iteration count is bounded by max_iterations.  FAST (the FP32-flux form): the residual by
 // err_eqn_fast and the convergence tests |dW| < tol |Wp|, |err| < tol |Wp| without the divisions;
 // FP64 throughout, equal to the plain form up to rounding.
-template <int NV, bool FAST = false>
-__device__ int u_to_p_onedw(const ZoneGeom& G, double gam, const double* U, double* P, int max_iterations, double tol)
+template <int NV, bool FAST = false, class AR>
+__device__ __forceinline__ int u_to_p_onedw(AR& ar, const ZoneGeom& G, double gam, const double* U, double* P, int max_iterations, double tol)
 {
     if (U[0] <= 0.) return ST_NEG_INPUT;
-    const double alpha = 1./sqrt(-G.gcon[0][0]);
+    const double alpha = ar.inv(ar.root(-G.gcon[0][0]));
     const double gdet = G.gdet;
-    const double a_over_g = alpha / gdet;
+    const double a_over_g = ar.div(alpha, gdet);
     const double D = U[0] * a_over_g;
     double Bcon[4] = {0., 0., 0., 0.};
     if (NV > 5) {
@@ -524,13 +594,13 @@ __device__ int u_to_p_onedw(const ZoneGeom& G, double gam, const double* U, doub
     const double Qtsq = dot4(Qcon, Qcov) + Qdotn*Qdotn;
     const double Ep = -Qdotn - D;
     int eflag = ST_SUCCESS;
-    const double gfac = (gam - 1) / gam;
+    const double gfac = ar.div(gam - 1, gam);
     auto residual = [&](double Wq) {
-        return FAST ? err_eqn_fast(gfac, Bsq, D, Ep, QdB, Qtsq, Wq, eflag) : err_eqn(gam, Bsq, D, Ep, QdB, Qtsq, Wq, eflag);
+        return FAST ? err_eqn_fast(ar, gfac, Bsq, D, Ep, QdB, Qtsq, Wq, eflag) : err_eqn(ar, gam, Bsq, D, Ep, QdB, Qtsq, Wq, eflag);
     };
     double Wp, err;
     {
-        const double gamma = lorentz(G.gcov, P[2], P[3], P[4]);
+        const double gamma = ar.root(lorentz_sq(G.gcov, P[2], P[3], P[4]));
         if (gamma < 1) return ST_BAD_UT;
         const double rho = P[0], u = P[1];
         Wp = (rho + u + (gam - 1) * u) * gamma * gamma - rho * gamma;
@@ -544,39 +614,46 @@ __device__ int u_to_p_onedw(const ZoneGeom& G, double gam, const double* U, doub
         const double errm = residual(Wpm);
         const double errp = residual(Wpp);
         if (FAST) {
-            const double idedW = (Wpp - Wpm) / (errp - errm);
-            const double dedW2 = (errp - 2. * err + errm) / (h*h);
-            const double f = kclip(0.5 * err * dedW2 * (idedW*idedW), -0.3, 0.3);
-            dW = kclip(-err * idedW / (1. - f), -0.5*Wp, 2.0*Wp);
+            const double idedW = ar.div(Wpp - Wpm, errp - errm);
+            const double dedW2 = ar.div(errp - 2. * err + errm, h*h);
+            const double f0 = 0.5 * err * dedW2 * (idedW*idedW), f = kclip(f0, -0.3, 0.3);
+            ar.see(f0);
+            dW = ar.div(-err * idedW, 1. - f);
         } else {
-            const double dedW = (errp - errm) / (Wpp - Wpm);
-            const double dedW2 = (errp - 2. * err + errm) / (h*h);
-            const double f = kclip(0.5 * err * dedW2 / (dedW*dedW), -0.3, 0.3);
-            dW = kclip(-err / dedW / (1. - f), -0.5*Wp, 2.0*Wp);
+            const double dedW = ar.div(errp - errm, Wpp - Wpm);
+            const double dedW2 = ar.div(errp - 2. * err + errm, h*h);
+            const double f0 = ar.div(0.5 * err * dedW2, dedW*dedW), f = kclip(f0, -0.3, 0.3);
+            ar.see(f0);
+            dW = ar.div(ar.div(-err, dedW), 1. - f);
         }
+        ar.see(dW);
+        dW = kclip(dW, -0.5*Wp, 2.0*Wp);
     }
     double Wp1 = Wp;
     double err1 = err;
     Wp += dW;
     err = residual(Wp);
     int iter = 0;
+#pragma unroll 1
     for (iter = 0; iter < max_iterations; iter++) {
-        dW = kclip((Wp1 - Wp) * err / (err - err1), -0.5*Wp, 2.0*Wp);
+        dW = ar.div((Wp1 - Wp) * err, err - err1);
+        ar.see(dW);
+        dW = kclip(dW, -0.5*Wp, 2.0*Wp);
         Wp1 = Wp;
         err1 = err;
         Wp += dW;
-        if (FAST ? fabs(dW) < tol * fabs(Wp) : fabs(dW / Wp) < tol) break;
+        if (FAST ? fabs(dW) < tol * fabs(Wp) : ratio_below(dW, Wp, tol)) break;
         err = residual(Wp);
-        if (FAST ? fabs(err) < tol * fabs(Wp) : fabs(err / Wp) < tol) break;
+        if (FAST ? fabs(err) < tol * fabs(Wp) : ratio_below(err, Wp, tol)) break;
     }
     if (iter == max_iterations) return ST_MAX_ITER;
     const double W = Wp + D;
     if (FAST) {
         // gamma = 1/ig with ig = rsqrt(1 + |utsq|), as in err_eqn_fast
         const double QdBsq = QdB * QdB, W2 = W * W, WB = W + Bsq;
-        const double utsq = -((W + WB) * QdBsq + W2 * Qtsq) / (QdBsq * (W + WB) + W2 * (Qtsq - WB * WB));
+        const double utsq = ar.div(-((W + WB) * QdBsq + W2 * Qtsq), QdBsq * (W + WB) + W2 * (Qtsq - WB * WB));
         if (utsq < -1.e-15 || utsq > 1.e7) return ST_BAD_UT;
-        const double ig = rsqrt(1. + fabs(utsq));
+        const double ig = ar.inv_root(1. + fabs(utsq));
         const double rho = D * ig;
         const double w = W * (ig * ig);
         const double p = (w - rho) * gfac;
@@ -586,28 +663,36 @@ __device__ int u_to_p_onedw(const ZoneGeom& G, double gam, const double* U, doub
         else if (u < 0) return ST_NEG_U;
         P[0] = rho;
         P[1] = u;
-        const double pre = 1. / (ig * WB), qw = QdB / W;
+        const double pre = ar.inv(ig * WB), qw = ar.div(QdB, W);
         P[2] = pre * (Qtcon[1] + qw * Bcon[1]);
         P[3] = pre * (Qtcon[2] + qw * Bcon[2]);
         P[4] = pre * (Qtcon[3] + qw * Bcon[3]);
         return ST_SUCCESS;
     }
-    const double gamma = lorentz_calc_w(Bsq, D, QdB, Qtsq, Wp);
+    const double gamma = lorentz_calc_w(ar, Bsq, D, QdB, Qtsq, Wp);
     if (gamma < 1) return ST_BAD_UT;
-    const double rho = D / gamma;
-    const double w = W / (gamma*gamma);
-    const double p = (w - rho) * (gam - 1) / gam;
+    const double rho = ar.div(D, gamma);
+    const double w = ar.div(W, gamma*gamma);
+    const double p = ar.div((w - rho) * (gam - 1), gam);
     const double u = w - (rho + p);
     if (rho < 0 && u < 0) return ST_NEG_RHOU;
     else if (rho < 0) return ST_NEG_RHO;
     else if (u < 0) return ST_NEG_U;
     P[0] = rho;
     P[1] = u;
-    const double pre = (gamma / (W + Bsq));
-    P[2] = pre * (Qtcon[1] + QdB * Bcon[1] / W);
-    P[3] = pre * (Qtcon[2] + QdB * Bcon[2] / W);
-    P[4] = pre * (Qtcon[3] + QdB * Bcon[3] / W);
+    const double pre = ar.div(gamma, W + Bsq);
+    const auto rW = ar.rcp(W);
+    P[2] = pre * (Qtcon[1] + ar.quot(QdB * Bcon[1], rW));
+    P[3] = pre * (Qtcon[2] + ar.quot(QdB * Bcon[2], rW));
+    P[4] = pre * (Qtcon[3] + ar.quot(QdB * Bcon[3], rW));
     return ST_SUCCESS;
+}
+
+template <int NV, bool FAST = false>
+__device__ int u_to_p_onedw(const ZoneGeom& G, double gam, const double* U, double* P, int max_iterations, double tol)
+{
+    Plain<double> ar;
+    return u_to_p_onedw<NV, FAST>(ar, G, gam, U, P, max_iterations, tol);
 }
 
 // ------------------------------------------------------------------ Kastaun inversion (FP64)
@@ -616,12 +701,15 @@ __device__ int u_to_p_onedw(const ZoneGeom& G, double gam, const double* U, doub
 // FFlag bits of the floors hit (FF_INVERTER_*), or ST_MAX_ITER with P untouched.
 enum { FF_INVERTER_RHO = 16384, FF_INVERTER_U = 32768, FF_INVERTER_GAMMA = 65536, FF_INVERTER_U_MAX = 131072 };
 
+template <class AR>
 struct KastaunResidual {
+    AR& ar;
     double D, q, bsq, bsq_rpsq, rsq, rbsq, v0sq, gam, rho_floor, e_floor, e_max;
+    __device__ __forceinline__ KastaunResidual(AR& a) : ar(a) {}
     bool used_density_floor, used_energy_floor, used_energy_max, used_gamma_max;
-    __device__ __forceinline__ double x_mu(double mu) const { return 1.0 / (1.0 + mu * bsq); }
-    __device__ __forceinline__ double rbarsq_mu(double mu, double x) const { return x * (x * rsq + mu * (1.0 + x) * rbsq); }
-    __device__ __forceinline__ double qbar_mu(double mu, double x) const
+    __device__ __forceinline__ double x_mu(double mu) { return ar.inv(1.0 + mu * bsq); }
+    __device__ __forceinline__ double rbarsq_mu(double mu, double x) { return x * (x * rsq + mu * (1.0 + x) * rbsq); }
+    __device__ __forceinline__ double qbar_mu(double mu, double x)
     {
         const double mux = mu * x;
         return q - 0.5 * (bsq + mux * mux * bsq_rpsq);
@@ -640,7 +728,7 @@ struct KastaunResidual {
     }
     __device__ __forceinline__ double ehat_mu(double mu, double qbar, double rbarsq, double vhatsq, double What)
     {
-        const double ehat_trial = What * (qbar - mu * rbarsq) + vhatsq * What * What / (1.0 + What);
+        const double ehat_trial = What * (qbar - mu * rbarsq) + ar.div(vhatsq * What * What, 1.0 + What);
         used_energy_floor = false;
         used_energy_max = false;
         if (ehat_trial <= e_floor) { used_energy_floor = true; return e_floor; }
@@ -653,24 +741,24 @@ struct KastaunResidual {
         const double rbarsq = rbarsq_mu(mu, x);
         const double qbar = qbar_mu(mu, x);
         const double vhatsq = vhatsq_mu(mu, rbarsq);
-        const double iWhat = sqrt(1.0 - vhatsq);
-        const double What = 1.0 / iWhat;
+        const double iWhat = ar.root(1.0 - vhatsq);
+        const double What = ar.inv(iWhat);
         const double rhohat = rhohat_mu(iWhat);
         const double ehat = ehat_mu(mu, qbar, rbarsq, vhatsq, What);
         const double Phat = ehat * rhohat * (gam - 1.0);
         const double hhat = rhohat * (1.0 + ehat) + Phat;
-        const double ahat = Phat / (hhat - Phat);
+        const double ahat = ar.div(Phat, hhat - Phat);
         const double nua = (1.0 + ahat) * (1.0 + ehat) * iWhat;
         const double nub = (1.0 + ahat) * (1.0 + qbar - mu * rbarsq);
         const double nuhat = kmax(nua, nub);
-        const double muhat = 1.0 / (nuhat + mu * rbarsq);
+        const double muhat = ar.inv(nuhat + mu * rbarsq);
         return mu - muhat;
     }
-    __device__ __forceinline__ double aux(double mu) const    // eq. 49
+    __device__ __forceinline__ double aux(double mu)          // eq. 49
     {
-        const double x = 1.0 / (1.0 + mu * bsq);
+        const double x = ar.inv(1.0 + mu * bsq);
         const double rbarsq = x * (rsq * x + mu * (1.0 + x) * rbsq);
-        return mu * sqrt(1.0 + rbarsq) - 1.0;
+        return mu * ar.root(1.0 + rbarsq) - 1.0;
     }
     // Illinois false position on [zm, zp] (kastaun.hpp:305-331, 343-368); iter at exit
     template <bool MASTER>
@@ -681,8 +769,10 @@ struct KastaunResidual {
         int iterations = max_iterations;
         if ((fabs(zm - zp) < tol) || ((fabs(fm) + fabs(fp)) < 2.0 * tol)) iterations = -1;
         double z = 0.5 * (zm + zp);
+#pragma unroll 1
         for (iter = 0; iter < iterations; ++iter) {
-            z = (zm * fp - zp * fm) / (fp - fm);
+            z = ar.div(zm * fp - zp * fm, fp - fm);
+            ar.see(z);
             const double fz = MASTER ? master(z) : aux(z);
             if ((fabs(zm - zp) < tol) || (fabs(fz) < tol)) break;
             if (fz * fp < 0.0) { zm = zp; fm = fp; zp = z; fp = fz; }
@@ -692,32 +782,34 @@ struct KastaunResidual {
     }
 };
 
-template <int NV>
-__device__ int u_to_p_kastaun(const ZoneGeom& G, double gam, const Prescription& fl, const double* U, double* P,
+template <int NV, class AR>
+__device__ __forceinline__ int u_to_p_kastaun(AR& ar, const ZoneGeom& G, double gam, const Prescription& fl, const double* U, double* P,
                               int max_iterations, double tol)
 {
-    const double alpha = 1. / sqrt(-G.gcon[0][0]);
-    const double a_over_g = alpha / G.gdet;
+    const double alpha = ar.inv(ar.root(-G.gcon[0][0]));
+    const double a_over_g = ar.div(alpha, G.gdet);
     const double D = U[0] * a_over_g;
     const double D_fl = kmax(D, fl.rho_min_const);
     const double Qcov[4] = {(U[1] - U[0]) * a_over_g, U[2] * a_over_g, U[3] * a_over_g, U[4] * a_over_g};
     const double ncov[4] = {-alpha, 0., 0., 0.};
     double ncon[4];
     raise4(G, ncov, ncon);
-    const double q = (-dot4(Qcov, ncon) - D) / D;
-    const double rcov[3] = {U[2] / U[0], U[3] / U[0], U[4] / U[0]};
+    const double q = ar.div(-dot4(Qcov, ncon) - D, D);
+    const auto rU0 = ar.rcp(U[0]);
+    const double rcov[3] = {ar.quot(U[2], rU0), ar.quot(U[3], rU0), ar.quot(U[4], rU0)};
     double rcon[3];
+    const auto rg00 = ar.rcp(G.gcon[0][0]);
 #pragma unroll
     for (int a = 0; a < 3; ++a)   // gamma^ij = g^ij - g^0i g^0j / g^00 (kastaun.hpp:250-262)
-        rcon[a] = ((G.gcon[a+1][1] - G.gcon[0][a+1]*G.gcon[0][1]/G.gcon[0][0])*rcov[0] +
-                   (G.gcon[a+1][2] - G.gcon[0][a+1]*G.gcon[0][2]/G.gcon[0][0])*rcov[1] +
-                   (G.gcon[a+1][3] - G.gcon[0][a+1]*G.gcon[0][3]/G.gcon[0][0])*rcov[2]);
+        rcon[a] = ((G.gcon[a+1][1] - ar.quot(G.gcon[0][a+1]*G.gcon[0][1], rg00))*rcov[0] +
+                   (G.gcon[a+1][2] - ar.quot(G.gcon[0][a+1]*G.gcon[0][2], rg00))*rcov[1] +
+                   (G.gcon[a+1][3] - ar.quot(G.gcon[0][a+1]*G.gcon[0][3], rg00))*rcov[2]);
     double rsq = 0.0;
 #pragma unroll
     for (int a = 0; a < 3; ++a) rsq += rcon[a] * rcov[a];
     double bsq = 0.0, bsq_rpsq = 0.0, rbsq = 0.0, bdotr = 0.0, bu[3] = {0.0, 0.0, 0.0};
     if (NV > 5) {
-        const double sD = 1.0 / sqrt(D_fl);
+        const double sD = ar.inv(ar.root(D_fl));
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
             bu[a] = (U[5 + a] * a_over_g) * sD;
@@ -732,20 +824,20 @@ __device__ int u_to_p_kastaun(const ZoneGeom& G, double gam, const Prescription&
         bsq_rpsq = bsq * rsq - rbsq;
     }
     const double zsq = rsq;
-    KastaunResidual res;
+    KastaunResidual<AR> res(ar);
     res.D = D; res.q = q; res.bsq = bsq; res.bsq_rpsq = bsq_rpsq; res.rsq = rsq; res.rbsq = rbsq;
-    res.v0sq = kmin(zsq / (1.0 + zsq), 1.0 - 1.0 / (fl.gamma_max * fl.gamma_max));
-    res.gam = gam; res.rho_floor = fl.rho_min_const; res.e_floor = fl.u_min_const / D_fl; res.e_max = fl.u_over_rho_max;
+    res.v0sq = kmin(ar.div(zsq, 1.0 + zsq), 1.0 - ar.inv(fl.gamma_max * fl.gamma_max));
+    res.gam = gam; res.rho_floor = fl.rho_min_const; res.e_floor = ar.div(fl.u_min_const, D_fl); res.e_max = fl.u_over_rho_max;
     res.used_density_floor = res.used_energy_floor = res.used_energy_max = res.used_gamma_max = false;
     int iter = 0;
-    const double zb = res.solve<false>(0., 1., max_iterations, tol, iter);
-    const double mu = res.solve<true>(0., zb, max_iterations, tol, iter);
+    const double zb = res.template solve<false>(0., 1., max_iterations, tol, iter);
+    const double mu = res.template solve<true>(0., zb, max_iterations, tol, iter);
     if (iter == max_iterations) return ST_MAX_ITER;
     const double x = res.x_mu(mu);
     const double rbarsq = res.rbarsq_mu(mu, x);
     const double vsq = res.vhatsq_mu(mu, rbarsq);
-    const double iW = sqrt(1.0 - vsq);
-    const double W = 1. / iW;
+    const double iW = ar.root(1.0 - vsq);
+    const double W = ar.inv(iW);
     P[0] = res.rhohat_mu(iW);
     const double qbar = res.qbar_mu(mu, x);
     P[1] = res.ehat_mu(mu, qbar, rbarsq, vsq, W) * P[0];
@@ -757,6 +849,14 @@ __device__ int u_to_p_kastaun(const ZoneGeom& G, double gam, const Prescription&
     if (res.used_gamma_max) fflag |= FF_INVERTER_GAMMA;
     if (res.used_energy_max) fflag |= FF_INVERTER_U_MAX;
     return fflag;
+}
+
+template <int NV>
+__device__ int u_to_p_kastaun(const ZoneGeom& G, double gam, const Prescription& fl, const double* U, double* P,
+                              int max_iterations, double tol)
+{
+    Plain<double> ar;
+    return u_to_p_kastaun<NV>(ar, G, gam, fl, U, P, max_iterations, tol);
 }
 
 // ------------------------------------------------------------------ floors (FP64)
@@ -796,20 +896,20 @@ __device__ __forceinline__ bool ktot_above(double gam, double rho, double u, dou
 // floors_functions.hpp:84-160
 // rhoflr_geom, uflr_geom: the geometric floor values of this zone (x3-independent, tabulated per
 // (j,i) at set-up with the same formula, floors_functions.hpp:96-104).  D returns the 4-vectors of P.
-template <int NV>
-__device__ int determine_floors(const ZoneGeom& G, const Prescription& f, double rhoflr_geom, double uflr_geom,
+template <int NV, class AR>
+__device__ __forceinline__ int determine_floors(AR& ar, const ZoneGeom& G, const Prescription& f, double rhoflr_geom, double uflr_geom,
                                 double gam, const double* P, double& rhoflr_max, double& uflr_max, FourVec<double>& D)
 {
     double gcon0[4] = {G.gcon[0][0], G.gcon[0][1], G.gcon[0][2], G.gcon[0][3]};
-    calc_4vecs<double, (NV > 5)>(G.gcov, G.gcon[0][0], gcon0, P, D);
+    calc_4vecs<double, (NV > 5)>(ar, G.gcov, G.gcon[0][0], gcon0, P, D);
     const double bsq = dot4(D.bcon, D.bcov);
-    const double rhoflr_b = bsq / f.bsq_over_rho_max;
-    const double uflr_b   = bsq / f.bsq_over_u_max;
+    const double rhoflr_b = ar.div(bsq, f.bsq_over_rho_max);
+    const double uflr_b   = ar.div(bsq, f.bsq_over_u_max);
     uflr_max = kmax(uflr_geom, uflr_b);
     const double rho = P[0], u = P[1];
     int fflag = 0;
     if (!f.temp_adjust_u) {
-        const double rhoflr_temp = kmax(u, uflr_max) / f.u_over_rho_max;
+        const double rhoflr_temp = ar.div(kmax(u, uflr_max), f.u_over_rho_max);
         fflag |= (rhoflr_temp > rho) * FF_TEMP;
         rhoflr_max = kmax(kmax(rhoflr_geom, rhoflr_b), rhoflr_temp);
     } else {
@@ -821,7 +921,7 @@ __device__ int determine_floors(const ZoneGeom& G, const Prescription& f, double
         fflag |= (rhoflr_b > rho) * FF_B_RHO;
         fflag |= (uflr_b > u) * FF_B_U;
     }
-    if (lorentz(G.gcov, P[2], P[3], P[4]) > f.gamma_max) fflag |= FF_GAMMA;
+    if (ar.root(lorentz_sq(G.gcov, P[2], P[3], P[4])) > f.gamma_max) fflag |= FF_GAMMA;
     if (ktot_above(gam, P[0], P[1], f.ktot_max)) fflag |= FF_KTOT;
     if (f.temp_adjust_u && (P[1] / P[0] > f.u_over_rho_max)) fflag |= FF_TEMP;
     return fflag;
@@ -848,8 +948,8 @@ __device__ __forceinline__ void apply_ceilings(const ZoneGeom& G, const Prescrip
 // floors_functions.hpp:174-179 (fluid), 181-252 (drift), 254-289 (normal observer)
 // D_pre: the 4-vectors of P on entry when the caller has them (determine_floors computed them from the
 // same P and geometry, so they are the ones the drift frame would compute), else NULL
-template <int NV>
-__device__ int apply_floors_frame(const ZoneGeom& G, int frame, double gam, double* P, double* U,
+template <int NV, class AR>
+__device__ __forceinline__ int apply_floors_frame(AR& ar, const ZoneGeom& G, int frame, double gam, double* P, double* U,
                                   double rhoflr_max, double uflr_max, int iter_max_nof,
                                   const FourVec<double>* D_pre = nullptr)
 {
@@ -858,7 +958,7 @@ __device__ int apply_floors_frame(const ZoneGeom& G, int frame, double gam, doub
         P[1] += kmax(0., uflr_max - P[1]);
         return 0;
     } else if (frame == 2) {
-        const double lapse2 = 1. / (-G.gcon[0][0]);
+        const double lapse2 = ar.inv(-G.gcon[0][0]);
         double beta[4] = {0., 0., 0., 0.};
         beta[1] = lapse2 * G.gcon[0][1];
         beta[2] = lapse2 * G.gcon[0][2];
@@ -874,13 +974,13 @@ __device__ int apply_floors_frame(const ZoneGeom& G, int frame, double gam, doub
 #pragma unroll
             for (int nu = 0; nu < 4; ++nu) Bcov[mu] += G.gcov[mu][nu] * Bcon[nu];
         const double Bsq   = kmax(dot4(Bcon, Bcov), 1e-20);
-        const double B_mag = sqrt(Bsq);
+        const double B_mag = ar.root(Bsq);
         FourVec<double> D;
         if (D_pre) {
             D = *D_pre;
         } else {
             double gcon0[4] = {G.gcon[0][0], G.gcon[0][1], G.gcon[0][2], G.gcon[0][3]};
-            calc_4vecs<double, (NV > 5)>(G.gcov, G.gcon[0][0], gcon0, P, D);
+            calc_4vecs<double, (NV > 5)>(ar, G.gcov, G.gcon[0][0], gcon0, P, D);
         }
         double Qcov[4];
         Qcov[0] = w_old * D.ucon[0] * D.ucov[0] + pg;
@@ -888,22 +988,23 @@ __device__ int apply_floors_frame(const ZoneGeom& G, int frame, double gam, doub
         Qcov[2] = w_old * D.ucon[0] * D.ucov[2];
         Qcov[3] = w_old * D.ucon[0] * D.ucov[3];
         const double QdotB = dot4(Bcon, Qcov);
-        double vpar = QdotB / (B_mag * w_old * D.ucon[0]*D.ucon[0]);
+        double vpar = ar.div(QdotB, B_mag * w_old * D.ucon[0]*D.ucon[0]);
         double ucon_dr[4] = {0., 0., 0., 0.};
-        ucon_dr[0] = 1. / sqrt(1. / (D.ucon[0]*D.ucon[0]) + vpar*vpar);
+        ucon_dr[0] = ar.inv(ar.root(ar.inv(D.ucon[0]*D.ucon[0]) + vpar*vpar));
+        const auto rBm = ar.rcp(B_mag);
 #pragma unroll
         for (int mu = 0; mu < 4; ++mu)
-            ucon_dr[mu] = D.ucon[mu] * (ucon_dr[0] / D.ucon[0]) - (vpar * Bcon[mu] * ucon_dr[0] / B_mag);
+            ucon_dr[mu] = D.ucon[mu] * ar.div(ucon_dr[0], D.ucon[0]) - ar.quot(vpar * Bcon[mu] * ucon_dr[0], rBm);
         P[0] = kmax(rho, rhoflr_max);
         P[1] = kmax(uu, uflr_max);
         const double pg_new = (gam - 1.) * P[1];
         const double w_new  = P[0] + P[1] + pg_new;
-        const double x = (2. * QdotB) / (B_mag * w_new * ucon_dr[0]);
-        vpar = x / (1 + sqrt(1 + x*x)) * (1. / ucon_dr[0]);
+        const double x = ar.div(2. * QdotB, B_mag * w_new * ucon_dr[0]);
+        vpar = ar.div(x, 1 + ar.root(1 + x*x)) * ar.inv(ucon_dr[0]);
         double uc[4];
-        uc[0] = 1. / sqrt(1/(ucon_dr[0]*ucon_dr[0]) - vpar*vpar);
+        uc[0] = ar.inv(ar.root(ar.inv(ucon_dr[0]*ucon_dr[0]) - vpar*vpar));
 #pragma unroll
-        for (int mu = 0; mu < 4; ++mu) uc[mu] = ucon_dr[mu] * (uc[0] / ucon_dr[0]) + (vpar * Bcon[mu] * uc[0] / B_mag);
+        for (int mu = 0; mu < 4; ++mu) uc[mu] = ucon_dr[mu] * ar.div(uc[0], ucon_dr[0]) + ar.quot(vpar * Bcon[mu] * uc[0], rBm);
         P[2] = uc[1] + (beta[1] * uc[0]);
         P[3] = uc[2] + (beta[2] * uc[0]);
         P[4] = uc[3] + (beta[3] * uc[0]);
@@ -914,7 +1015,7 @@ __device__ int apply_floors_frame(const ZoneGeom& G, int frame, double gam, doub
         double Pa[8] = {rho_add, u_add, 0., 0., 0., 0., 0., 0.};
         FourVec<double> D;
         double gcon0[4] = {G.gcon[0][0], G.gcon[0][1], G.gcon[0][2], G.gcon[0][3]};
-        calc_4vecs<double, true>(G.gcov, G.gcon[0][0], gcon0, Pa, D);
+        calc_4vecs<double, true>(ar, G.gcov, G.gcon[0][0], gcon0, Pa, D);
         const double rho_ut = rho_add * D.ucon[0] * G.gdet;
         double mhd[4];
         calc_tensor<double, true>(rho_add, u_add, (gam - 1) * u_add, D, 0, mhd);
@@ -925,7 +1026,7 @@ __device__ int apply_floors_frame(const ZoneGeom& G, int frame, double gam, doub
         U[2] += mhd[1] * G.gdet;
         U[3] += mhd[2] * G.gdet;
         U[4] += mhd[3] * G.gdet;
-        return u_to_p_onedw<NV>(G, gam, U, P, iter_max_nof, 1e-8);
+        return u_to_p_onedw<NV>(ar, G, gam, U, P, iter_max_nof, 1e-8);
     }
 }
 

@@ -894,7 +894,8 @@ __global__ void __launch_bounds__(128) k_emhd_dudt(Dims d, DevGeom g, Phys ph, E
             du_[p] = -du / vol;
         }
         double db[3];
-        ct_divergence<double>(d, ph, F1, F2, F3, c, j, db);
+        Plain<double> ar;
+        ct_divergence<double>(ar, ar.rcp(ph.dx1*ph.dx2*ph.dx3), d, ph, F1, F2, F3, c, j, db);
 #pragma unroll
         for (int v = 0; v < 3; ++v) du_[5 + v] = db[v];
         if (!ph.cart_minkowski) {
@@ -1397,9 +1398,10 @@ __global__ void __launch_bounds__(128) k_emhd_floors(Dims d, DevGeom g, Phys ph,
     const Prescription& fl = floors_at(ph, g, j, i);
     double rf, uf;
     FourVec<double> D;
-    const int ff = determine_floors<8>(G, fl, __ldg(g.floor_rho + cg), __ldg(g.floor_u + cg), ph.gam, Pz, rf, uf, D);
+    Plain<double> ar;
+    const int ff = determine_floors<8>(ar, G, fl, __ldg(g.floor_rho + cg), __ldg(g.floor_u + cg), ph.gam, Pz, rf, uf, D);
     if (ff) {
-        apply_floors_frame<8>(G, ph.frame, ph.gam, Pz, Uz, rf, uf, 8, &D);
+        apply_floors_frame<8>(ar, G, ph.frame, ph.gam, Pz, Uz, rf, uf, 8, &D);
         apply_ceilings(G, fl, ph.gam, Pz);
 #pragma unroll
         for (int p = 0; p < 5; ++p) P.v[p][c] = Pz[p];

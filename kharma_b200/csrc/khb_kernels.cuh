@@ -49,6 +49,27 @@ __device__ __forceinline__ bool box_cell(const Box& b, unsigned blk, int& i, int
     return true;
 }
 
+// Loads and stores at 32-bit byte offsets from a base all threads share: the base stays in uniform
+// registers and one offset per stencil point serves every variable, where 64-bit element indices cost
+// two to four integer instructions per access.  An offset spans one variable of a block: the largest
+// block that fits the memory of a GPU has below 2^29 zones.
+template <typename T>
+__device__ __forceinline__ T ldo(const T* base, unsigned off)
+{
+    return __ldg(reinterpret_cast<const T*>(reinterpret_cast<const char*>(base) + off));
+}
+// ... through the coherent path, for arrays the same launch also writes
+template <typename T>
+__device__ __forceinline__ T lds(const T* base, unsigned off)
+{
+    return *reinterpret_cast<const T*>(reinterpret_cast<const char*>(base) + off);
+}
+template <typename T>
+__device__ __forceinline__ void sto(T* base, unsigned off, T v)
+{
+    *reinterpret_cast<T*>(reinterpret_cast<char*>(base) + off) = v;
+}
+
 // Load the centre geometry of zone (j,i)
 // SYM: the upper triangles only, mirrored (10 values per metric held in registers instead of 16).
 // The host tables are symmetric to rounding, not bit for bit, so only the FP32-flux form, which has
@@ -56,16 +77,16 @@ __device__ __forceinline__ bool box_cell(const Box& b, unsigned blk, int& i, int
 template <bool SYM = false>
 __device__ __forceinline__ void load_zone_geom(const DevGeom& g, int j, int i, ZoneGeom& G)
 {
-    const long long gi = (long long)j*g.G1 + i;
+    const unsigned gi = (unsigned)(j*g.G1 + i) * 8u;
 #pragma unroll
     for (int m = 0; m < 16; ++m) {
         const int r = m/4, q = m%4;
         if (SYM && q < r) continue;
-        G.gcov[r][q] = __ldg(g.gcov[3] + m*g.gs + gi);
-        G.gcon[r][q] = __ldg(g.gcon[3] + m*g.gs + gi);
+        G.gcov[r][q] = ldo(g.gcov[3] + m*g.gs, gi);
+        G.gcon[r][q] = ldo(g.gcon[3] + m*g.gs, gi);
         if (SYM) { G.gcov[q][r] = G.gcov[r][q]; G.gcon[q][r] = G.gcon[r][q]; }
     }
-    G.gdet = __ldg(g.gdet[3] + gi);
+    G.gdet = ldo(g.gdet[3], gi);
 }
 
 // The floor prescription of zone (j, i): the inner one inside floors_switch_r when radius-dependent
@@ -77,13 +98,19 @@ __device__ __forceinline__ const Prescription& floors_at(const Phys& ph, const D
 }
 
 // Flux::p_to_u for one zone (all NV conserved variables), flux_functions.hpp:343-352
-template <int NV>
-__device__ __forceinline__ void p_to_u_zone(const ZoneGeom& G, double gam, const double* P, double* U)
+template <int NV, class AR>
+__device__ __forceinline__ void p_to_u_zone(AR& ar, const ZoneGeom& G, double gam, const double* P, double* U)
 {
     FourVec<double> D;
     const double gcon0[4] = {G.gcon[0][0], G.gcon[0][1], G.gcon[0][2], G.gcon[0][3]};
-    calc_4vecs<double, (NV > 5)>(G.gcov, G.gcon[0][0], gcon0, P, D);
+    calc_4vecs<double, (NV > 5)>(ar, G.gcov, G.gcon[0][0], gcon0, P, D);
     prim_to_flux<double, NV>(P, D, gam, G.gdet, 0, U);
+}
+template <int NV>
+__device__ __forceinline__ void p_to_u_zone(const ZoneGeom& G, double gam, const double* P, double* U)
+{
+    Plain<double> ar;
+    p_to_u_zone<NV>(ar, G, gam, P, U);
 }
 
 // ===================================================================================== fluxes
@@ -101,30 +128,31 @@ template <> struct FaceTables<float> {
 };
 
 // Resident 128-thread blocks per SM requested from the compiler for each kernel (register caps
-// of 65536 / (128 x blocks)), chosen by measurement on B200: FP64 faces 6 blocks along x1/x2 and 5
-// along x3 (with the L2 prefetch of each zone's primitives; 5 and 4 before it), FP32 faces 8, the update half of the zone pass 4 (FP64 fluxes; no spills) or 5 (FP32
-// fluxes) and its inversion half 5 (6 in the FP32-flux form, whose zone pass holds the metric's
-// upper triangles only).  Each can be overridden at build time.
+// of 65536 / (128 x blocks)), chosen by measurement on B200 (128^3 torus, us per step).  With the
+// branch-free divisions the compiler overlaps the chains of a face or zone, and registers buy more than
+// warps: FP64 faces 4 blocks (128 registers, no spills; 5 blocks cost 20%, 3 nothing), FP64 update half
+// 3 (2350 against 2398 at 4 and 2503 at 5), FP64 cell half 4, both halves of the FP32-flux form 5 (1668
+// against 1711 at 4), FP32 faces 8.  Each can be overridden at build time.
 #ifndef KHB_FLUX64_MINB
-#define KHB_FLUX64_MINB 6
+#define KHB_FLUX64_MINB 4
 #endif
 #ifndef KHB_FLUX64_X3_MINB
-#define KHB_FLUX64_X3_MINB 5
+#define KHB_FLUX64_X3_MINB 4
 #endif
 #ifndef KHB_FLUX32_MINB
 #define KHB_FLUX32_MINB 8
 #endif
 #ifndef KHB_ZONE_UPDATE_MINB
-#define KHB_ZONE_UPDATE_MINB 4
+#define KHB_ZONE_UPDATE_MINB 3
 #endif
 #ifndef KHB_ZONE_UPDATE32_MINB
 #define KHB_ZONE_UPDATE32_MINB 5
 #endif
 #ifndef KHB_ZONE_CELL_MINB
-#define KHB_ZONE_CELL_MINB 5
+#define KHB_ZONE_CELL_MINB 4
 #endif
 #ifndef KHB_ZONE_CELL32_MINB
-#define KHB_ZONE_CELL32_MINB 6
+#define KHB_ZONE_CELL32_MINB 5
 #endif
 #ifndef KHB_ZONE_INV_MINB
 #define KHB_ZONE_INV_MINB 6
@@ -146,35 +174,50 @@ template <int MODE_, typename FT> struct ZoneMinBlocks {
 
 // L2 prefetch of the line holding p (PTX prefetch.global.L2: a hint, no register result)
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+template <typename T>
+__device__ __forceinline__ void prefetch_o(const T* base, unsigned off) { prefetch_l2(reinterpret_cast<const char*>(base) + off); }
 
-template <int DIR, int RECON, int NV, typename R, typename FT>
-__device__ __forceinline__ void flux_face(const Dims& d, const DevGeom& g, const Phys& ph, const khb_fields& P,
+// One face with the divisions and roots of policy AR; false where AR's operand checks failed (the
+// values written are then to be replaced).
+// What bounds a FP64 face is instruction issue and the FP64 pipe: with the compiler's divisions and 64-bit
+// addresses a linear-MC face took 3420 warp instructions, a third of them FP64, at 64% issue; with
+// Exact64 and 32-bit offsets 1660, 59% of them FP64, at 57% issue and 66% of the FP64 pipe (96^3 torus:
+// 152 to 85 us along x1, 173 to 84 along x3).
+template <int DIR, int RECON, int NV, typename R, typename FT, class AR>
+__device__ __forceinline__ bool flux_face_by(const Dims& d, const DevGeom& g, const Phys& ph, const khb_fields& P,
                                           FT* __restrict__ F, FT* __restrict__ ctop, int i, int j, int k)
 {
     constexpr int dir = DIR;
+    AR ar;
     const long long c = kchk(d, ((long long)k*d.n2 + j)*d.n1 + i, d.N, CHK_FLUX_STORE);
     const long long st = (dir == 1) ? 1 : ((dir == 2) ? d.sj : d.sk);
     const int loc = dir - 1;
     const R gam = (R)ph.gam;
 
+    // byte offsets of the six stencil zones in a state array, and of the face in a flux array
+    const unsigned oc = (unsigned)c * 8u;
+    const unsigned o0 = (unsigned)kchk(d, c - 3*st, d.N, CHK_FLUX_STENCIL) * 8u, o1 = (unsigned)kchk(d, c - 2*st, d.N, CHK_FLUX_STENCIL) * 8u;
+    const unsigned o2 = (unsigned)kchk(d, c - st, d.N, CHK_FLUX_STENCIL) * 8u, o4 = (unsigned)kchk(d, c + st, d.N, CHK_FLUX_STENCIL) * 8u;
+    const unsigned o5 = (unsigned)kchk(d, c + 2*st, d.N, CHK_FLUX_STENCIL) * 8u;
+    const unsigned of = (unsigned)c * (unsigned)sizeof(FT);
     // FP64 faces: start the zone's own primitives towards L2 first (measured: 2.6% off the FP64
     // step; the FP32 faces, issue bound, do not gain)
     if (sizeof(R) == 8) {
 #pragma unroll
-        for (int p = 0; p < NV; ++p) prefetch_l2(P.v[p] + c);
+        for (int p = 0; p < NV; ++p) prefetch_o(P.v[p], oc);
     }
     // geometry at the face
-    const long long gi = kchk(d, (long long)j*g.G1 + i, g.gs, CHK_GEOM);
+    const unsigned gi = (unsigned)kchk(d, (long long)j*g.G1 + i, g.gs, CHK_GEOM) * (unsigned)sizeof(R);
     const auto* tcov = FaceTables<R>::gcov(g, loc);
     const auto* tcon = FaceTables<R>::gcon(g, loc);
     R gcov[4][4];
 #pragma unroll
-    for (int m = 0; m < 16; ++m) gcov[m/4][m%4] = (R)__ldg(tcov + m*g.gs + gi);
+    for (int m = 0; m < 16; ++m) gcov[m/4][m%4] = ldo(tcov + m*g.gs, gi);
     R gcon0[4];
 #pragma unroll
-    for (int m = 0; m < 4; ++m) gcon0[m] = (R)__ldg(tcon + m*g.gs + gi);
-    const R gcondd = (R)__ldg(tcon + (dir*4 + dir)*g.gs + gi);
-    const R gdet = (R)__ldg(FaceTables<R>::gdet(g, loc) + gi);
+    for (int m = 0; m < 4; ++m) gcon0[m] = ldo(tcon + m*g.gs, gi);
+    const R gcondd = ldo(tcon + (dir*4 + dir)*g.gs, gi);
+    const R gdet = ldo(FaceTables<R>::gdet(g, loc), gi);
 
     // reconstruction: left state = right face of zone c-st, right state = left face of zone c
     R Pl[NV], Pr[NV];
@@ -195,18 +238,21 @@ __device__ __forceinline__ void flux_face(const Dims& d, const DevGeom& g, const
 #pragma unroll
     for (int p = 0; p < NV; ++p) {
         const double* q = P.v[p];
-        const R x0 = (R)__ldg(q + kchk(d, c - 3*st, d.N, CHK_FLUX_STENCIL)), x1 = (R)__ldg(q + kchk(d, c - 2*st, d.N, CHK_FLUX_STENCIL));
-        const R x2 = (R)__ldg(q + kchk(d, c - st, d.N, CHK_FLUX_STENCIL)), x3 = (R)__ldg(q + c);
-        const R x4 = (R)__ldg(q + kchk(d, c + st, d.N, CHK_FLUX_STENCIL)), x5 = (R)__ldg(q + kchk(d, c + 2*st, d.N, CHK_FLUX_STENCIL));
+        const R x0 = (R)ldo(q, o0), x1 = (R)ldo(q, o1), x2 = (R)ldo(q, o2);
+        const R x3 = (R)ldo(q, oc), x4 = (R)ldo(q, o4), x5 = (R)ldo(q, o5);
+        if (RECON == RECON_WENO5 || RECON == RECON_WENO5X) {
+            // bounds what the weights divide (recon_right)
+            ar.bounded(x0); ar.bounded(x1); ar.bounded(x2); ar.bounded(x3); ar.bounded(x4); ar.bounded(x5);
+        }
         if (RECON == RECON_EXTRA) {
             Pl[p] = recon_extra<R>(ph.recon_extra, true, x0, x1, x2, x3, x4);
             Pr[p] = recon_extra<R>(ph.recon_extra, false, x1, x2, x3, x4, x5);
         } else if (RECON == RECON_WENO5X) {
-            Pl[p] = mc_l ? recon_right<RECON_MC, R>(x0, x1, x2, x3, x4) : recon_right<RECON_WENO5, R>(x0, x1, x2, x3, x4);
-            Pr[p] = mc_r ? recon_left<RECON_MC, R>(x1, x2, x3, x4, x5) : recon_left<RECON_WENO5, R>(x1, x2, x3, x4, x5);
+            Pl[p] = mc_l ? recon_right<RECON_MC, R>(ar, x0, x1, x2, x3, x4) : recon_right<RECON_WENO5, R>(ar, x0, x1, x2, x3, x4);
+            Pr[p] = mc_r ? recon_left<RECON_MC, R>(ar, x1, x2, x3, x4, x5) : recon_left<RECON_WENO5, R>(ar, x1, x2, x3, x4, x5);
         } else {
-            Pl[p] = recon_right<RECON, R>(x0, x1, x2, x3, x4);
-            Pr[p] = recon_left<RECON, R>(x1, x2, x3, x4, x5);
+            Pl[p] = recon_right<RECON, R>(ar, x0, x1, x2, x3, x4);
+            Pr[p] = recon_left<RECON, R>(ar, x1, x2, x3, x4, x5);
         }
     }
     constexpr bool HIGH = (RECON == RECON_WENO5X || RECON == RECON_EXTRA);
@@ -222,11 +268,10 @@ __device__ __forceinline__ void flux_face(const Dims& d, const DevGeom& g, const
 #pragma unroll
             for (int p = 0; p < NV; ++p) {
                 const double* q = P.v[p];
-                const R x0 = (R)__ldg(q + kchk(d, c - 3*st, d.N, CHK_FLUX_STENCIL)), x1 = (R)__ldg(q + kchk(d, c - 2*st, d.N, CHK_FLUX_STENCIL));
-                const R x2 = (R)__ldg(q + kchk(d, c - st, d.N, CHK_FLUX_STENCIL)), x3 = (R)__ldg(q + c);
-                const R x4 = (R)__ldg(q + kchk(d, c + st, d.N, CHK_FLUX_STENCIL)), x5 = (R)__ldg(q + kchk(d, c + 2*st, d.N, CHK_FLUX_STENCIL));
-                Pl[p] = recon_right<RECON_PPM, R>(x0, x1, x2, x3, x4);
-                Pr[p] = recon_left<RECON_PPM, R>(x1, x2, x3, x4, x5);
+                const R x0 = (R)ldo(q, o0), x1 = (R)ldo(q, o1), x2 = (R)ldo(q, o2);
+                const R x3 = (R)ldo(q, oc), x4 = (R)ldo(q, o4), x5 = (R)ldo(q, o5);
+                Pl[p] = recon_right<RECON_PPM, R>(ar, x0, x1, x2, x3, x4);
+                Pr[p] = recon_left<RECON_PPM, R>(ar, x1, x2, x3, x4, x5);
             }
         }
     }
@@ -235,14 +280,14 @@ __device__ __forceinline__ void flux_face(const Dims& d, const DevGeom& g, const
     FourVec<R> D;
     R Ul[NV], Fl[NV], Ur[NV], Fr[NV];
     R cmaxL, cminL, cmaxR, cminR;
-    calc_4vecs<R, HAS_B>(gcov, gcon0[0], gcon0, Pl, D);
+    calc_4vecs<R, HAS_B>(ar, gcov, gcon0[0], gcon0, Pl, D);
     prim_to_flux<R, NV>(Pl, D, gam, gdet, 0, Ul);
     prim_to_flux<R, NV>(Pl, D, gam, gdet, dir, Fl);
-    vchar<R, HAS_B>(Pl, D, gam, gcon0[0], gcon0[dir], gcondd, dir, cmaxL, cminL);
-    calc_4vecs<R, HAS_B>(gcov, gcon0[0], gcon0, Pr, D);
+    vchar<R, HAS_B>(ar, Pl, D, gam, gcon0[0], gcon0[dir], gcondd, dir, cmaxL, cminL);
+    calc_4vecs<R, HAS_B>(ar, gcov, gcon0[0], gcon0, Pr, D);
     prim_to_flux<R, NV>(Pr, D, gam, gdet, 0, Ur);
     prim_to_flux<R, NV>(Pr, D, gam, gdet, dir, Fr);
-    vchar<R, HAS_B>(Pr, D, gam, gcon0[0], gcon0[dir], gcondd, dir, cmaxR, cminR);
+    vchar<R, HAS_B>(ar, Pr, D, gam, gcon0[0], gcon0[dir], gcondd, dir, cmaxR, cminR);
     // get_flux.hpp:274-275, 330-331
     const R cmax = kmax(kmax(R(0), cmaxL), cmaxR);
     const R cmin = -kmin(kmin(R(0), cminL), cminR);
@@ -250,18 +295,40 @@ __device__ __forceinline__ void flux_face(const Dims& d, const DevGeom& g, const
         const R ctp = kmax(cmax, cmin);
 #pragma unroll
         for (int p = 0; p < NV; ++p)
-            F[p*d.N + c] = (FT)(R(0.5) * (Fl[p] + Fr[p] - ctp * (Ur[p] - Ul[p])));
+            sto(F + p*d.N, of, (FT)(R(0.5) * (Fl[p] + Fr[p] - ctp * (Ur[p] - Ul[p]))));
     } else {
+        const auto rsum = ar.rcp(cmax + cmin);
 #pragma unroll
         for (int p = 0; p < NV; ++p)
-            F[p*d.N + c] = (FT)((cmax*Fl[p] + cmin*Fr[p] - cmax*cmin*(Ur[p] - Ul[p])) / (cmax + cmin));
+            sto(F + p*d.N, of, (FT)ar.quot(cmax*Fl[p] + cmin*Fr[p] - cmax*cmin*(Ur[p] - Ul[p]), rsum));
     }
-    ctop[c] = (FT)kmax(cmax, cmin);
+    sto(ctop, of, (FT)kmax(cmax, cmin));
+    // both sides' states run into the fluxes of density and energy (a NaN anywhere makes them one)
+    ar.see(Fl[0] + Fr[0]); ar.see(Ur[0] - Ul[0]);
+    ar.see(Fl[1] + Fr[1]); ar.see(Ur[1] - Ul[1]);
+    return ar.ok();
+}
+
+// The same face with the operators themselves, out of line (FP64 faces whose operands failed the checks)
+template <int DIR, int RECON, int NV, typename R, typename FT>
+__device__ __noinline__ void flux_face_plain(const Dims& d, const DevGeom& g, const Phys& ph, const khb_fields& P,
+                                             FT* __restrict__ F, FT* __restrict__ ctop, int i, int j, int k)
+{
+    flux_face_by<DIR, RECON, NV, R, FT, Plain<R>>(d, g, ph, P, F, ctop, i, j, k);
+}
+
+template <int DIR, int RECON, int NV, typename R, typename FT>
+__device__ __forceinline__ void flux_face(const Dims& d, const DevGeom& g, const Phys& ph, const khb_fields& P,
+                                          FT* __restrict__ F, FT* __restrict__ ctop, int i, int j, int k)
+{
+    if (!flux_face_by<DIR, RECON, NV, R, FT, typename FastArith<R>::type>(d, g, ph, P, F, ctop, i, j, k))
+        flux_face_plain<DIR, RECON, NV, R, FT>(d, g, ph, P, F, ctop, i, j, k);
 }
 
 template <int DIR, int RECON, int NV, typename R, typename FT>
 __global__ void __launch_bounds__(128, FluxMinBlocks<R, DIR>::value)
-k_flux(Dims d, DevGeom g, Phys ph, khb_fields P, FT* __restrict__ F, FT* __restrict__ ctop, Box bx)
+k_flux(const __grid_constant__ Dims d, const __grid_constant__ DevGeom g, const __grid_constant__ Phys ph,
+       const __grid_constant__ khb_fields P, FT* __restrict__ F, FT* __restrict__ ctop, Box bx)
 {
     int i, j, k;
     if (!box_cell(bx, blockIdx.x, i, j, k)) return;
@@ -336,64 +403,64 @@ __global__ void __launch_bounds__(128) k_fix_tasks(const FixTask<FT>* __restrict
 // Raw flux, as double
 template <typename FT>
 __device__ __forceinline__ double ldf(const FT* F, long long x) { return (double)__ldg(F + x); }
+// ... at a byte offset
+template <typename FT>
+__device__ __forceinline__ double ldfo(const FT* F, unsigned x) { return (double)ldo(F, x); }
 
 // Divergence of the B fluxes with flux-CT applied on the fly (b_flux_ct.cpp:307-370): corner EMFs
 // from the raw B fluxes in FT arithmetic, the face B fluxes from the EMFs, then -div over the zone.
 // F1..F3 hold nvar-major fluxes with the B components in slots 5-7 (stride d.N).
-template <typename FT>
-__device__ __forceinline__ void ct_divergence(const Dims& d, const Phys& ph, const FT* F1, const FT* F2, const FT* F3,
-                                              long long c, int j, double dudt_b[3])
+template <typename FT, class AR>
+__device__ __forceinline__ void ct_divergence(AR& ar, const typename AR::Rcp& rvol, const Dims& d, const Phys& ph,
+                                              const FT* F1, const FT* F2, const FT* F3, long long c, int j, double dudt_b[3])
 {
-    const long long N = d.N, sj = d.sj, sk = d.sk;
+    const long long N = d.N;
     const double a1 = ph.dx2*ph.dx3, a2 = ph.dx1*ph.dx3, a3 = ph.dx1*ph.dx2;
-    const double vol = ph.dx1*ph.dx2*ph.dx3;
+    // byte offsets of the zone and its neighbours' strides in a flux array
+    constexpr unsigned s1 = sizeof(FT);
+    const unsigned x0 = (unsigned)c * s1, sj = (unsigned)d.sj * s1, sk = (unsigned)d.sk * s1;
     double fb[3][3][2];   // [face dir][B component][lo/hi face]
     if (d.ndim >= 2) {
-        const long long B1 = 5*N, B2 = 6*N, B3 = 7*N;
-        // corner EMFs; the checked build verifies the furthest reaches of each (x itself, x - sj or
-        // x - sk, x - 1) against the field's extent
-        auto e3 = [&](long long x) -> FT {
-            x = kchk(d, x, N, CHK_ZONE_CT); kchk(d, x - sj, N, CHK_ZONE_CT); kchk(d, x - 1, N, CHK_ZONE_CT);
-            return (FT)0.25 * (__ldg(F1 + B2 + x) + __ldg(F1 + B2 + x - sj) - __ldg(F2 + B1 + x) - __ldg(F2 + B1 + x - 1));
+        const FT* F1B2 = F1 + 6*N; const FT* F1B3 = F1 + 7*N;
+        const FT* F2B1 = F2 + 5*N; const FT* F2B3 = F2 + 7*N;
+        const FT* F3B1 = F3 + 5*N; const FT* F3B2 = F3 + 6*N;
+        // corner EMFs
+        auto at = [&](const FT* F, unsigned x) -> FT {
+            return ldo(F, KHB_BOUNDS_CHECK ? (unsigned)kchk(d, x / s1, N, CHK_ZONE_CT) * s1 : x);
         };
-        auto e1 = [&](long long x) -> FT {
-            x = kchk(d, x, N, CHK_ZONE_CT); kchk(d, x - sk, N, CHK_ZONE_CT); kchk(d, x - sj, N, CHK_ZONE_CT);
-            return (FT)0.25 * (__ldg(F2 + B3 + x) + __ldg(F2 + B3 + x - sk) - __ldg(F3 + B2 + x) - __ldg(F3 + B2 + x - sj));
-        };
-        auto e2 = [&](long long x) -> FT {
-            x = kchk(d, x, N, CHK_ZONE_CT); kchk(d, x - 1, N, CHK_ZONE_CT); kchk(d, x - sk, N, CHK_ZONE_CT);
-            return (FT)0.25 * (__ldg(F3 + B1 + x) + __ldg(F3 + B1 + x - 1) - __ldg(F1 + B3 + x) - __ldg(F1 + B3 + x - sk));
-        };
+        auto e3 = [&](unsigned x) -> FT { return (FT)0.25 * (at(F1B2, x) + at(F1B2, x - sj) - at(F2B1, x) - at(F2B1, x - s1)); };
+        auto e1 = [&](unsigned x) -> FT { return (FT)0.25 * (at(F2B3, x) + at(F2B3, x - sk) - at(F3B2, x) - at(F3B2, x - sj)); };
+        auto e2 = [&](unsigned x) -> FT { return (FT)0.25 * (at(F3B1, x) + at(F3B1, x - s1) - at(F1B3, x) - at(F1B3, x - sk)); };
         const bool d3 = d.ndim > 2;
         // X1 faces i (lo) and i+1 (hi)
         fb[0][0][0] = 0.; fb[0][0][1] = 0.;
-        fb[0][1][0] = (double)((FT)0.5 * (e3(c) + e3(c + sj)));
-        fb[0][1][1] = (double)((FT)0.5 * (e3(c + 1) + e3(c + 1 + sj)));
-        fb[0][2][0] = d3 ? (double)((FT)-0.5 * (e2(c) + e2(c + sk))) : ldf(F1, B3 + c);
-        fb[0][2][1] = d3 ? (double)((FT)-0.5 * (e2(c + 1) + e2(c + 1 + sk))) : ldf(F1, B3 + c + 1);
+        fb[0][1][0] = (double)((FT)0.5 * (e3(x0) + e3(x0 + sj)));
+        fb[0][1][1] = (double)((FT)0.5 * (e3(x0 + s1) + e3(x0 + s1 + sj)));
+        fb[0][2][0] = d3 ? (double)((FT)-0.5 * (e2(x0) + e2(x0 + sk))) : ldfo(F1B3, x0);
+        fb[0][2][1] = d3 ? (double)((FT)-0.5 * (e2(x0 + s1) + e2(x0 + s1 + sk))) : ldfo(F1B3, x0 + s1);
         // X2 faces j, j+1
-        fb[1][0][0] = (double)((FT)-0.5 * (e3(c) + e3(c + 1)));
-        fb[1][0][1] = (double)((FT)-0.5 * (e3(c + sj) + e3(c + sj + 1)));
+        fb[1][0][0] = (double)((FT)-0.5 * (e3(x0) + e3(x0 + s1)));
+        fb[1][0][1] = (double)((FT)-0.5 * (e3(x0 + sj) + e3(x0 + sj + s1)));
         fb[1][1][0] = 0.; fb[1][1][1] = 0.;
-        fb[1][2][0] = d3 ? (double)((FT)0.5 * (e1(c) + e1(c + sk))) : ldf(F2, B3 + c);
-        fb[1][2][1] = d3 ? (double)((FT)0.5 * (e1(c + sj) + e1(c + sj + sk))) : ldf(F2, B3 + c + sj);
+        fb[1][2][0] = d3 ? (double)((FT)0.5 * (e1(x0) + e1(x0 + sk))) : ldfo(F2B3, x0);
+        fb[1][2][1] = d3 ? (double)((FT)0.5 * (e1(x0 + sj) + e1(x0 + sj + sk))) : ldfo(F2B3, x0 + sj);
         // KBoundaries zero_polar_flux after flux-CT (boundaries.cpp:672-684)
         if (ph.zero_polar_flux) {
             if (j == d.js && phys_face(d.bc[2])) { fb[1][0][0] = 0.; fb[1][1][0] = 0.; fb[1][2][0] = 0.; }
             if (j == d.je && phys_face(d.bc[3])) { fb[1][0][1] = 0.; fb[1][1][1] = 0.; fb[1][2][1] = 0.; }
         }
         if (d3) {
-            fb[2][0][0] = (double)((FT)0.5 * (e2(c) + e2(c + 1)));
-            fb[2][0][1] = (double)((FT)0.5 * (e2(c + sk) + e2(c + sk + 1)));
-            fb[2][1][0] = (double)((FT)-0.5 * (e1(c) + e1(c + sj)));
-            fb[2][1][1] = (double)((FT)-0.5 * (e1(c + sk) + e1(c + sk + sj)));
+            fb[2][0][0] = (double)((FT)0.5 * (e2(x0) + e2(x0 + s1)));
+            fb[2][0][1] = (double)((FT)0.5 * (e2(x0 + sk) + e2(x0 + sk + s1)));
+            fb[2][1][0] = (double)((FT)-0.5 * (e1(x0) + e1(x0 + sj)));
+            fb[2][1][1] = (double)((FT)-0.5 * (e1(x0 + sk) + e1(x0 + sk + sj)));
             fb[2][2][0] = 0.; fb[2][2][1] = 0.;
         }
     } else {
 #pragma unroll
         for (int v = 0; v < 3; ++v) {
-            fb[0][v][0] = ldf(F1, (5 + v)*N + c);
-            fb[0][v][1] = ldf(F1, (5 + v)*N + c + 1);
+            fb[0][v][0] = ldfo(F1 + (5 + v)*N, x0);
+            fb[0][v][1] = ldfo(F1 + (5 + v)*N, x0 + s1);
         }
     }
 #pragma unroll
@@ -401,21 +468,24 @@ __device__ __forceinline__ void ct_divergence(const Dims& d, const Phys& ph, con
         double du = (a1 * fb[0][v][1] - a1 * fb[0][v][0]);
         if (d.ndim >= 2) du += a2 * fb[1][v][1] - a2 * fb[1][v][0];
         if (d.ndim == 3) du += a3 * fb[2][v][1] - a3 * fb[2][v][0];
-        dudt_b[v] = -du / vol;
+        dudt_b[v] = ar.quot(-du, rvol);
     }
 }
 
 // B_CT::BlockUtoP for one zone (b_ct.cpp:172-181): the zone B^i as the average of its two faces'
 // B^i = Bf / sqrt(-g)(face); along an inactive direction the single face's value
-__device__ __forceinline__ void ct_zone_b(const Dims& d, const DevGeom& g, const double* const Bf[3], long long c,
+template <class AR>
+__device__ __forceinline__ void ct_zone_b(AR& ar, const Dims& d, const DevGeom& g, const double* const Bf[3], long long c,
                                           int j, int i, double Bp[3])
 {
-    const long long gi = (long long)j*g.G1 + i;
-    Bp[0] = (__ldg(Bf[0] + c) / __ldg(g.gdet[0] + gi) + __ldg(Bf[0] + c + 1) / __ldg(g.gdet[0] + gi + 1)) / 2;
-    Bp[1] = (d.ndim > 1) ? (__ldg(Bf[1] + c) / __ldg(g.gdet[1] + gi) + __ldg(Bf[1] + c + d.sj) / __ldg(g.gdet[1] + gi + g.G1)) / 2
-                         : __ldg(Bf[1] + c) / __ldg(g.gdet[1] + gi);
-    Bp[2] = (d.ndim > 2) ? (__ldg(Bf[2] + c) / __ldg(g.gdet[2] + gi) + __ldg(Bf[2] + c + d.sk) / __ldg(g.gdet[2] + gi)) / 2
-                         : __ldg(Bf[2] + c) / __ldg(g.gdet[2] + gi);
+    const unsigned x = (unsigned)c * 8u, gi = (unsigned)(j*g.G1 + i) * 8u;
+    Bp[0] = (ar.div(ldo(Bf[0], x), ldo(g.gdet[0], gi)) + ar.div(ldo(Bf[0], x + 8u), ldo(g.gdet[0], gi + 8u))) / 2;
+    Bp[1] = ar.div(ldo(Bf[1], x), ldo(g.gdet[1], gi));
+    if (d.ndim > 1)
+        Bp[1] = (Bp[1] + ar.div(ldo(Bf[1], x + (unsigned)d.sj * 8u), ldo(g.gdet[1], gi + (unsigned)g.G1 * 8u))) / 2;
+    const auto r3 = ar.rcp(ldo(g.gdet[2], gi));
+    Bp[2] = ar.quot(ldo(Bf[2], x), r3);
+    if (d.ndim > 2) Bp[2] = (Bp[2] + ar.quot(ldo(Bf[2], x + (unsigned)d.sk * 8u), r3)) / 2;
 }
 
 // ct_zone_b for any zone of the block: the last layer of a direction (i = n1-1, j = n2-1, k = n3-1)
@@ -434,16 +504,17 @@ __device__ __forceinline__ void ct_zone_b_edge(const Dims& d, const DevGeom& g, 
 
 // The geometric source of one zone (flux.cpp:413-441): new_du[lam] = sum over mu, nu of
 // T^mu_nu gdet Gamma^nu_lam mu for the UU and U1-U3 components, from the zone's primitives Ps
-template <int NV>
-__device__ __forceinline__ void geo_source(const Dims& d, const DevGeom& g, const ZoneGeom& G, double gam,
+template <int NV, class AR>
+__device__ __forceinline__ void geo_source(AR& ar, const Dims& d, const DevGeom& g, const ZoneGeom& G, double gam,
                                            const double* Ps, int j, int i, double new_du[4])
 {
     FourVec<double> D;
     const double gcon0[4] = {G.gcon[0][0], G.gcon[0][1], G.gcon[0][2], G.gcon[0][3]};
-    calc_4vecs<double, (NV > 5)>(G.gcov, G.gcon[0][0], gcon0, Ps, D);
+    calc_4vecs<double, (NV > 5)>(ar, G.gcov, G.gcon[0][0], gcon0, Ps, D);
 #pragma unroll
     for (int lam = 0; lam < 4; ++lam) new_du[lam] = 0.;
-    const long long cg = (long long)j*g.n1 + i, cs = (long long)(d.n2)*g.n1;
+    const unsigned cg = (unsigned)(j*g.n1 + i) * 8u;
+    const long long cs = (long long)(d.n2)*g.n1;
 #pragma unroll
     for (int mu = 0; mu < 4; ++mu) {
         double Tmu[4];
@@ -452,199 +523,210 @@ __device__ __forceinline__ void geo_source(const Dims& d, const DevGeom& g, cons
         for (int nu = 0; nu < 4; ++nu)
 #pragma unroll
             for (int lam = 0; lam < 4; ++lam)
-                new_du[lam] += Tmu[nu] * __ldg(g.gdet_conn + ((nu*4 + lam)*4 + mu)*cs + cg);
+                new_du[lam] += Tmu[nu] * ldo(g.gdet_conn + ((nu*4 + lam)*4 + mu)*cs, cg);
     }
 }
 
 // MODE: compile-time mask of M_* steps (0: take the mask from the arguments at run time).  The
 // CFL reduction (M_DT) is always a run-time choice.
+// One zone of the zone pass with the divisions and roots of policy AR; false, with nothing written,
+// where AR's operand checks failed
+template <int NV, typename FT, int MODE, class AR>
+__device__ __forceinline__ bool zone_by(const Dims& d, const DevGeom& g, const Phys& ph, const ZoneArgs<FT>& a,
+                                        int i, int j, int k)
+{
+    AR ar;
+    const int mode = MODE ? (MODE | (a.mode & M_DT)) : a.mode;
+    const long long c = kchk(d, ((long long)k*d.n2 + j)*d.n1 + i, d.N, CHK_ZONE_FLUX);
+    const long long N = d.N;
+    const double gam = ph.gam;
+    kchk(d, c + 1, N, CHK_ZONE_FLUX);
+    if (d.ndim >= 2) kchk(d, c + d.sj, N, CHK_ZONE_FLUX);
+    if (d.ndim == 3) kchk(d, c + d.sk, N, CHK_ZONE_FLUX);
+    kchk(d, (long long)j*g.G1 + i, g.gs, CHK_GEOM);
+    // byte offsets of the zone in a state and in a flux array, strides in a flux array
+    const unsigned oc = (unsigned)c * 8u;
+    constexpr unsigned s1 = sizeof(FT);
+    const unsigned of = (unsigned)c * s1, sj = (unsigned)d.sj * s1, sk = (unsigned)d.sk * s1;
+    ZoneGeom G;
+    load_zone_geom<(sizeof(FT) == 4)>(g, j, i, G);
+
+    double U[NV], P[NV];
+    if (mode & M_UPDATE) {
+        // ---- flux divergence (Parthenon FluxDivHelper) with flux-CT B fluxes
+        const double a1 = ph.dx2*ph.dx3, a2 = ph.dx1*ph.dx3, a3 = ph.dx1*ph.dx2;
+        const auto rvol = ar.rcp(ph.dx1*ph.dx2*ph.dx3);
+        const FT* F1 = a.F[0]; const FT* F2 = a.F[1]; const FT* F3 = a.F[2];
+        double dudt[NV];
+        constexpr int NH = 5;
+#pragma unroll
+        for (int p = 0; p < NH; ++p) {
+            double du = (a1 * ldfo(F1 + p*N, of + s1) - a1 * ldfo(F1 + p*N, of));
+            if (d.ndim >= 2) du += a2 * ldfo(F2 + p*N, of + sj) - a2 * ldfo(F2 + p*N, of);
+            if (d.ndim == 3) du += a3 * ldfo(F3 + p*N, of + sk) - a3 * ldfo(F3 + p*N, of);
+            dudt[p] = ar.quot(-du, rvol);
+        }
+        if (NV > 5) {
+            double dudt_b[3] = {0., 0., 0.};
+            // with B_CT the zone B follows the faces (below) and has no flux divergence
+            if (!(mode & M_BCT)) ct_divergence<FT>(ar, rvol, d, ph, F1, F2, F3, c, j, dudt_b);
+#pragma unroll
+            for (int v = 0; v < 3; ++v) dudt[5 + v] = dudt_b[v];
+        }
+        // ---- geometric source, flux.cpp:395-444
+        if (!ph.cart_minkowski) {
+            double Ps[NV];
+#pragma unroll
+            for (int p = 0; p < NV; ++p) Ps[p] = ldo(a.Ps.v[p], oc);
+            double new_du[4];
+            geo_source<NV>(ar, d, g, G, gam, Ps, j, i, new_du);
+            dudt[1] += new_du[0];
+            dudt[2] += new_du[1];
+            dudt[3] += new_du[2];
+            dudt[4] += new_du[3];
+        }
+        // ---- RK combination (Parthenon WeightedSumData twice, kharma_driver.cpp:339-387)
+        const double bdt = a.dt_dev ? a.beta * __ldg(a.dt_dev) : a.bdt;
+#pragma unroll
+        for (int p = 0; p < NV; ++p) {
+            double x = a.g0 * ldo(a.Us.v[p], oc) + a.g1 * ldo(a.U0.v[p], oc);
+            U[p] = 1.0 * x + bdt * dudt[p];
+        }
+        if (NV > 5 && (mode & M_BCT)) {
+            // B_CT::BlockUtoP on the updated faces: sqrt(-g) B^i at the zone centre
+            double Bp[3];
+            ct_zone_b(ar, d, g, a.Bf, c, j, i, Bp);
+#pragma unroll
+            for (int v = 0; v < 3; ++v) U[5 + v] = Bp[v] * G.gdet;
+        }
+    } else {
+#pragma unroll
+        for (int p = 0; p < NV; ++p) U[p] = lds(a.Us.v[p], oc);
+        if (NV > 5 && (MODE & M_GHOSTB) && (mode & M_BCT)) {
+            // B_CT::BlockUtoP over the entire block before the inversion (b_ct.cpp:160-188)
+            double Bp[3];
+            ct_zone_b_edge(d, g, a.Bf, c, j, i, k, Bp);
+#pragma unroll
+            for (int v = 0; v < 3; ++v) U[5 + v] = Bp[v] * G.gdet;
+        }
+    }
+
+    int pflag = 0, fflag = 0;
+    FourVec<double> D;
+    bool have_D = false;
+#pragma unroll
+    for (int p = 0; p < NV; ++p) P[p] = lds(a.Ps.v[p], oc);
+    if (mode & M_UTOP) {
+        // inverter.cpp:163-181 then b_flux_ct.cpp:196-217
+        const int pf = (mode & M_KASTAUN) ? u_to_p_kastaun<NV>(ar, G, gam, floors_at(ph, g, j, i), U, P, ph.iter_max, ph.err_tol)
+                                          : u_to_p_onedw<NV, (sizeof(FT) == 4)>(ar, G, gam, U, P, ph.iter_max, ph.err_tol);
+        pflag = pf % FF_GEOM_RHO;
+        fflag = (pf / FF_GEOM_RHO) * FF_GEOM_RHO;
+        if (NV > 5) {
+            if (mode & M_BCT) {
+                double Bp[3];
+                if (MODE & M_GHOSTB) ct_zone_b_edge(d, g, a.Bf, c, j, i, k, Bp);
+                else ct_zone_b(ar, d, g, a.Bf, c, j, i, Bp);
+#pragma unroll
+                for (int v = 0; v < 3; ++v) P[5 + v] = Bp[v];
+            } else {
+                const auto rg = ar.rcp(G.gdet);
+#pragma unroll
+                for (int v = 0; v < 3; ++v) P[5 + v] = ar.quot(U[5 + v], rg);
+            }
+        }
+    } else {
+        pflag = a.pflag[c];
+        fflag = a.fflag[c];
+    }
+    if ((mode & M_UTOP) && (mode & (M_FLOORS | M_PTOU))) {
+        // reload the metric for floors and P->U instead of holding it through the inversion
+        // (the compiler barrier keeps the reload; measured 0.4% / 1.3% off the FP64 / FP32 step)
+        asm volatile("" ::: "memory");
+        load_zone_geom<(sizeof(FT) == 4)>(g, j, i, G);
+    }
+    if ((mode & M_FLOORS) && ph.floors_on) {
+        // floors.cpp:215-229 and floors_impl.hpp:77-125
+        double rf, uf;
+        const long long cg = (long long)j*g.n1 + i;
+        const Prescription& fl = floors_at(ph, g, j, i);
+        fflag |= determine_floors<NV>(ar, G, fl, __ldg(g.floor_rho + cg), __ldg(g.floor_u + cg), gam, P, rf, uf, D);
+        if (fflag) {
+            // mixed frames (floors_impl.hpp:84-106): by radius, or by min(rho, u)/b^2 of the
+            // state before the floors
+            int frame = ph.frame;
+            if (frame == KHB_FRAME_MIXED_FLUID_NORMAL) {
+                frame = (__ldg(g.rcen + cg) > ph.frame_switch_r) ? KHB_FRAME_FLUID : KHB_FRAME_NORMAL;
+            } else if (frame == KHB_FRAME_MIXED_NORMAL_DRIFT) {
+                const double mag_switch = kmin(P[0], P[1]) / dot4(D.bcon, D.bcov);
+                frame = (mag_switch < ph.frame_switch_beta) ? KHB_FRAME_DRIFT : KHB_FRAME_NORMAL;
+            }
+            const int pl = apply_floors_frame<NV>(ar, G, frame, gam, P, U, rf, uf, 8, &D);
+            if (pl) pflag = pl;
+            apply_ceilings(G, fl, gam, P);
+            // the fluid part of U(P) after the floors; the lock-step P->U below computes the same
+            // values from the same P, so it is formed here only when that step is not part of the pass
+            if (!(mode & M_PTOU)) {
+                double Ut[NV];
+                p_to_u_zone<NV>(ar, G, gam, P, Ut);
+#pragma unroll
+                for (int p = 0; p < 5; ++p) U[p] = Ut[p];
+            }
+        } else {
+            have_D = true;   // P is unchanged: its 4-vectors serve the P->U below
+        }
+    }
+    if (mode & M_PTOU) {
+        if (have_D) prim_to_flux<double, NV>(P, D, gam, G.gdet, 0, U);
+        else p_to_u_zone<NV>(ar, G, gam, P, U);
+    }
+    // a NaN in any primitive or 4-vector is one in the energy; the field's quotients stand alone
+    ar.see(U[1]);
+    ar.see(P[1]);
+    if (NV > 5) {
+#pragma unroll
+        for (int v = 0; v < 3; ++v) { ar.see(P[2 + v]); ar.see(P[5 + v]); ar.see(U[5 + v]); }
+    }
+    if (!ar.ok()) return false;
+
+    if (mode & (M_UPDATE | M_FLOORS | M_PTOU)) {
+#pragma unroll
+        for (int p = 0; p < NV; ++p) sto(a.Uout.v[p], oc, U[p]);
+    }
+    if (mode & (M_UTOP | M_FLOORS)) {
+#pragma unroll
+        for (int p = 0; p < NV; ++p) sto(a.Pout.v[p], oc, P[p]);
+        a.pflag[c] = pflag;
+        a.fflag[c] = fflag;
+    }
+    if ((mode & M_FAILLIST) && pflag > 0) {
+        const int slot = atomicAdd(a.fail_count, 1);
+        a.fail_list[slot] = (int)c;
+    }
+    return true;
+}
+
+// The same zone with the operators themselves, out of line (zones whose operands failed the checks)
+template <int NV, typename FT, int MODE>
+__device__ __noinline__ void zone_plain(const Dims& d, const DevGeom& g, const Phys& ph, const ZoneArgs<FT>& a,
+                                        int i, int j, int k)
+{
+    zone_by<NV, FT, MODE, Plain<double>>(d, g, ph, a, i, j, k);
+}
+
 // One zone of the zone pass; returns the zone's timestep for the CFL minimum (DBL_MAX if none)
 template <int NV, typename FT, int MODE>
 __device__ __forceinline__ double zone_body(const Dims& d, const DevGeom& g, const Phys& ph, const ZoneArgs<FT>& a,
                                             int i, int j, int k)
 {
-    const int mode = MODE ? (MODE | (a.mode & M_DT)) : a.mode;
-    double ndt_zone = 1.7976931348623157e308;
-    {
-        const long long c = kchk(d, ((long long)k*d.n2 + j)*d.n1 + i, d.N, CHK_ZONE_FLUX);
-        const long long N = d.N, sj = d.sj, sk = d.sk;
-        const double gam = ph.gam;
-        kchk(d, c + 1, N, CHK_ZONE_FLUX);
-        if (d.ndim >= 2) kchk(d, c + sj, N, CHK_ZONE_FLUX);
-        if (d.ndim == 3) kchk(d, c + sk, N, CHK_ZONE_FLUX);
-        kchk(d, (long long)j*g.G1 + i, g.gs, CHK_GEOM);
-        ZoneGeom G;
-        load_zone_geom<(sizeof(FT) == 4)>(g, j, i, G);
-
-        double U[NV], P[NV];
-        if (mode & M_UPDATE) {
-            // ---- flux divergence (Parthenon FluxDivHelper) with flux-CT B fluxes
-            const double a1 = ph.dx2*ph.dx3, a2 = ph.dx1*ph.dx3, a3 = ph.dx1*ph.dx2;
-            const double vol = ph.dx1*ph.dx2*ph.dx3;
-            const FT* F1 = a.F[0]; const FT* F2 = a.F[1]; const FT* F3 = a.F[2];
-            // the zone's own values come from DRAM: start them towards L2 before the register-bound
-            // loads below (no registers held, results unchanged)
-#pragma unroll
-            for (int p = 0; p < NV; ++p) {
-                prefetch_l2(a.Us.v[p] + c);
-                prefetch_l2(a.U0.v[p] + c);
-                prefetch_l2(F1 + p*N + c);
-                if (d.ndim >= 2) prefetch_l2(F2 + p*N + c);
-                if (d.ndim == 3) prefetch_l2(F3 + p*N + c);
-                if (!ph.cart_minkowski) prefetch_l2(a.Ps.v[p] + c);
-                if (sizeof(FT) == 8) {
-                    // FP64 fluxes: the upper x2/x3 faces too (measured 0.5% off the FP64 step; the FP32
-                    // form, whose flux lines are half as many, loses 4% with them)
-                    if (d.ndim >= 2) prefetch_l2(F2 + p*N + c + sj);
-                    if (d.ndim == 3) prefetch_l2(F3 + p*N + c + sk);
-                }
-            }
-            double dudt[NV];
-            constexpr int NH = 5;
-#pragma unroll
-            for (int p = 0; p < NH; ++p) {
-                double du = (a1 * ldf(F1, p*N + c + 1) - a1 * ldf(F1, p*N + c));
-                if (d.ndim >= 2) du += a2 * ldf(F2, p*N + c + sj) - a2 * ldf(F2, p*N + c);
-                if (d.ndim == 3) du += a3 * ldf(F3, p*N + c + sk) - a3 * ldf(F3, p*N + c);
-                dudt[p] = -du / vol;
-            }
-            if (NV > 5) {
-                double dudt_b[3] = {0., 0., 0.};
-                // with B_CT the zone B follows the faces (below) and has no flux divergence
-                if (!(mode & M_BCT)) ct_divergence<FT>(d, ph, F1, F2, F3, c, j, dudt_b);
-#pragma unroll
-                for (int v = 0; v < 3; ++v) dudt[5 + v] = dudt_b[v];
-            }
-            // ---- geometric source, flux.cpp:395-444
-            if (!ph.cart_minkowski) {
-                double Ps[NV];
-#pragma unroll
-                for (int p = 0; p < NV; ++p) Ps[p] = __ldg(a.Ps.v[p] + c);
-                double new_du[4];
-                geo_source<NV>(d, g, G, gam, Ps, j, i, new_du);
-                dudt[1] += new_du[0];
-                dudt[2] += new_du[1];
-                dudt[3] += new_du[2];
-                dudt[4] += new_du[3];
-            }
-            // ---- RK combination (Parthenon WeightedSumData twice, kharma_driver.cpp:339-387)
-            const double bdt = a.dt_dev ? a.beta * __ldg(a.dt_dev) : a.bdt;
-#pragma unroll
-            for (int p = 0; p < NV; ++p) {
-                double x = a.g0 * __ldg(a.Us.v[p] + c) + a.g1 * __ldg(a.U0.v[p] + c);
-                U[p] = 1.0 * x + bdt * dudt[p];
-            }
-            if (NV > 5 && (mode & M_BCT)) {
-                // B_CT::BlockUtoP on the updated faces: sqrt(-g) B^i at the zone centre
-                double Bp[3];
-                ct_zone_b(d, g, a.Bf, c, j, i, Bp);
-#pragma unroll
-                for (int v = 0; v < 3; ++v) U[5 + v] = Bp[v] * G.gdet;
-            }
-        } else {
-#pragma unroll
-            for (int p = 0; p < NV; ++p) U[p] = a.Us.v[p][c];
-            if (NV > 5 && (MODE & M_GHOSTB) && (mode & M_BCT)) {
-                // B_CT::BlockUtoP over the entire block before the inversion (b_ct.cpp:160-188)
-                double Bp[3];
-                ct_zone_b_edge(d, g, a.Bf, c, j, i, k, Bp);
-#pragma unroll
-                for (int v = 0; v < 3; ++v) U[5 + v] = Bp[v] * G.gdet;
-            }
-        }
-
-        int pflag = 0, fflag = 0;
-        FourVec<double> D;
-        bool have_D = false;
-#pragma unroll
-        for (int p = 0; p < NV; ++p) P[p] = a.Ps.v[p][c];
-        if (mode & M_UTOP) {
-            // inverter.cpp:163-181 then b_flux_ct.cpp:196-217
-            const int pf = (mode & M_KASTAUN) ? u_to_p_kastaun<NV>(G, gam, floors_at(ph, g, j, i), U, P, ph.iter_max, ph.err_tol)
-                                              : u_to_p_onedw<NV, (sizeof(FT) == 4)>(G, gam, U, P, ph.iter_max, ph.err_tol);
-            pflag = pf % FF_GEOM_RHO;
-            fflag = (pf / FF_GEOM_RHO) * FF_GEOM_RHO;
-            if (NV > 5) {
-                if (mode & M_BCT) {
-                    double Bp[3];
-                    if (MODE & M_GHOSTB) ct_zone_b_edge(d, g, a.Bf, c, j, i, k, Bp);
-                    else ct_zone_b(d, g, a.Bf, c, j, i, Bp);
-#pragma unroll
-                    for (int v = 0; v < 3; ++v) P[5 + v] = Bp[v];
-                } else {
-#pragma unroll
-                    for (int v = 0; v < 3; ++v) P[5 + v] = U[5 + v] / G.gdet;
-                }
-            }
-        } else {
-            pflag = a.pflag[c];
-            fflag = a.fflag[c];
-        }
-        if ((mode & M_UTOP) && (mode & (M_FLOORS | M_PTOU))) {
-            // reload the metric for floors and P->U instead of holding it through the inversion
-            // (the compiler barrier keeps the reload; measured 0.4% / 1.3% off the FP64 / FP32 step)
-            asm volatile("" ::: "memory");
-            load_zone_geom<(sizeof(FT) == 4)>(g, j, i, G);
-        }
-        if ((mode & M_FLOORS) && ph.floors_on) {
-            // floors.cpp:215-229 and floors_impl.hpp:77-125
-            double rf, uf;
-            const long long cg = (long long)j*g.n1 + i;
-            const Prescription& fl = floors_at(ph, g, j, i);
-            fflag |= determine_floors<NV>(G, fl, __ldg(g.floor_rho + cg), __ldg(g.floor_u + cg), gam, P, rf, uf, D);
-            if (fflag) {
-                // mixed frames (floors_impl.hpp:84-106): by radius, or by min(rho, u)/b^2 of the
-                // state before the floors
-                int frame = ph.frame;
-                if (frame == KHB_FRAME_MIXED_FLUID_NORMAL) {
-                    frame = (__ldg(g.rcen + cg) > ph.frame_switch_r) ? KHB_FRAME_FLUID : KHB_FRAME_NORMAL;
-                } else if (frame == KHB_FRAME_MIXED_NORMAL_DRIFT) {
-                    const double mag_switch = kmin(P[0], P[1]) / dot4(D.bcon, D.bcov);
-                    frame = (mag_switch < ph.frame_switch_beta) ? KHB_FRAME_DRIFT : KHB_FRAME_NORMAL;
-                }
-                const int pl = apply_floors_frame<NV>(G, frame, gam, P, U, rf, uf, 8, &D);
-                if (pl) pflag = pl;
-                apply_ceilings(G, fl, gam, P);
-                // the fluid part of U(P) after the floors; the lock-step P->U below computes the same
-                // values from the same P, so it is formed here only when that step is not part of the pass
-                if (!(mode & M_PTOU)) {
-                    double Ut[NV];
-                    p_to_u_zone<NV>(G, gam, P, Ut);
-#pragma unroll
-                    for (int p = 0; p < 5; ++p) U[p] = Ut[p];
-                }
-            } else {
-                have_D = true;   // P is unchanged: its 4-vectors serve the P->U below
-            }
-        }
-        if (mode & M_PTOU) {
-            if (have_D) prim_to_flux<double, NV>(P, D, gam, G.gdet, 0, U);
-            else p_to_u_zone<NV>(G, gam, P, U);
-        }
-
-        if (mode & (M_UPDATE | M_FLOORS | M_PTOU)) {
-#pragma unroll
-            for (int p = 0; p < NV; ++p) a.Uout.v[p][c] = U[p];
-        }
-        if (mode & (M_UTOP | M_FLOORS)) {
-#pragma unroll
-            for (int p = 0; p < NV; ++p) a.Pout.v[p][c] = P[p];
-            a.pflag[c] = pflag;
-            a.fflag[c] = fflag;
-        }
-        if ((mode & M_FAILLIST) && pflag > 0) {
-            const int slot = atomicAdd(a.fail_count, 1);
-            a.fail_list[slot] = (int)c;
-        }
-        if (mode & M_DT) {
-            // grmhd.cpp:313-328
-            const double c1 = kmax((double)a.ctop[0][c], 0.0), c2 = kmax((double)a.ctop[1][c], 0.0);
-            const double c3 = kmax((double)a.ctop[2][c], 0.0);
-            const double z = 1.0 / (1 / (ph.dx1 / c1) + 1 / (ph.dx2 / c2) + 1 / (ph.dx3 * 1 / c3));
-            if (!isnan(z)) ndt_zone = z;
-        }
-    }
-    return ndt_zone;
+    if (!zone_by<NV, FT, MODE, Exact64>(d, g, ph, a, i, j, k)) zone_plain<NV, FT, MODE>(d, g, ph, a, i, j, k);
+    if (!(a.mode & M_DT)) return 1.7976931348623157e308;
+    // grmhd.cpp:313-328
+    const long long c = kchk(d, ((long long)k*d.n2 + j)*d.n1 + i, d.N, CHK_ZONE_FLUX);
+    const double c1 = kmax((double)a.ctop[0][c], 0.0), c2 = kmax((double)a.ctop[1][c], 0.0);
+    const double c3 = kmax((double)a.ctop[2][c], 0.0);
+    const double z = 1.0 / (1 / (ph.dx1 / c1) + 1 / (ph.dx2 / c2) + 1 / (ph.dx3 * 1 / c3));
+    return isnan(z) ? 1.7976931348623157e308 : z;
 }
 
 // Block minimum of the zone timesteps by warp shuffles, then one atomic per block on the bit
@@ -665,7 +747,8 @@ __device__ __forceinline__ void block_min_ndt(double v, unsigned long long* word
 
 template <int NV, typename FT, int MODE>
 __global__ void __launch_bounds__(128, ZoneMinBlocks<MODE, FT>::value)
-k_zone(Dims d, DevGeom g, Phys ph, ZoneArgs<FT> a, Box bx)
+k_zone(const __grid_constant__ Dims d, const __grid_constant__ DevGeom g, const __grid_constant__ Phys ph,
+       const __grid_constant__ ZoneArgs<FT> a, Box bx)
 {
     int i, j, k;
     double ndt_zone = 1.7976931348623157e308;
@@ -706,7 +789,8 @@ __global__ void __launch_bounds__(128) k_fofc_guess(Dims d, DevGeom g, Phys ph, 
     // fofc/use_source_term: the guess also takes the geometric source of P_s (kharma_driver.cpp:308-312)
     if (ph.fofc_source && !ph.cart_minkowski) {
         double new_du[4];
-        geo_source<NV>(d, g, G, ph.gam, Pg, j, i, new_du);
+        Plain<double> ar;
+        geo_source<NV>(ar, d, g, G, ph.gam, Pg, j, i, new_du);
 #pragma unroll
         for (int v = 0; v < 4; ++v) dudt[1 + v] += new_du[v];
     }
@@ -726,7 +810,8 @@ __global__ void __launch_bounds__(128) k_fofc_guess(Dims d, DevGeom g, Phys ph, 
         const long long cg = (long long)j*g.n1 + i;
         double rf, uf;
         FourVec<double> D;
-        ff |= determine_floors<NV>(G, floors_at(ph, g, j, i), __ldg(g.floor_rho + cg), __ldg(g.floor_u + cg), ph.gam, Pg, rf, uf, D);
+        Plain<double> ar;
+        ff |= determine_floors<NV>(ar, G, floors_at(ph, g, j, i), __ldg(g.floor_rho + cg), __ldg(g.floor_u + cg), ph.gam, Pg, rf, uf, D);
     }
     const bool eh = ph.spherical && __ldg(g.rcen + (long long)j*g.n1 + i) < ph.fofc_r_mark;
     flag[c] = (ff != 0 || eh) ? 1 : 0;

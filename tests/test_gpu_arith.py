@@ -1,0 +1,79 @@
+"""The branch-free divisions and square roots of the FP64 kernels (csrc/khb_arith.cuh) at the ends of their
+range, where the kernels repeat a face or zone with the operators: against the oracle, which divides as
+IEEE 754 does.  Cartesian modes have no library transcendental on the path, so values of ordinary size
+are compared bit for bit (zeros of either sign alike); where a field runs down to the smallest doubles,
+whose last bits are not promised, each variable to 1e-12 of its largest."""
+import dataclasses
+
+import numpy as np
+import pytest
+import torch
+
+from kharma_b200 import problems
+from kharma_b200.block import Block
+from kharma_b200.spec import mhdmodes_spec
+
+from test_gpu_parity import RTOL, rel_err
+
+pytestmark = pytest.mark.gpu
+
+
+def tail(P):
+    """The field falls by powers of ten along x1 from 1 to below the smallest normal double."""
+    n1 = P.shape[-1]
+    P[5:8] *= 10.0 ** np.linspace(0, -320, n1)
+    return P
+
+
+def still(P):
+    """No motion, no field, uniform: every difference, 4-vector and field quotient has a zero in it."""
+    P[0], P[1], P[2:] = 1.0, 0.5, 0.0
+    return P
+
+
+def creeping(P):
+    """Velocities whose squares are an ulp of one: Lorentz factors and lapses of 1 - 2^-53 and 1 + 2^-52,
+    divisors with all significand bits set."""
+    rng = np.random.Generator(np.random.PCG64(3))
+    P[2:5] = 1.5e-8 * rng.uniform(-1, 1, P[2:5].shape)
+    P[5:8] *= 1e-8
+    return P
+
+
+def wide(P):
+    """Densities and pressures over 200 powers of ten."""
+    P[0:2] *= 10.0 ** np.linspace(-100, 100, P.shape[-1])
+    P[5:8] = 0.0
+    return P
+
+
+STATES = {"tail": tail, "still": still, "creeping": creeping, "wide": wide}
+
+
+@pytest.mark.parametrize("recon", ["linear_mc", "weno5", "ppm"])
+@pytest.mark.parametrize("inverter", ["onedw", "kastaun"])
+@pytest.mark.parametrize("state", list(STATES))
+def test_range_ends(oracle_mod, state, inverter, recon):
+    spec = dataclasses.replace(mhdmodes_spec(19, 13, 8, recon=recon, riemann="hlle" if recon == "ppm" else "llf"),
+                               inverter=inverter)
+    if inverter == "kastaun":
+        spec = dataclasses.replace(spec, iter_max=25, err_tol=1e-12)
+    P0 = STATES[state](problems.mhdmodes(spec, 3, amp=1e-2))
+    o = oracle_mod.Oracle(spec)
+    b = Block(spec, geometry=o.geometry())
+    b.set_prims(P0)
+    Po, Uo = o.init_state(P0)
+    for _ in range(2):
+        pf, ff, _, _ = o.step(Po, Uo, 1e-4)
+        b.step(1e-4)
+    torch.cuda.synchronize()
+    P, U = b.P.cpu().numpy(), b.U.cpu().numpy()
+    sl = spec.interior
+    assert np.array_equal(b.pflag.cpu().numpy()[sl], pf[sl].astype(np.int32))
+    assert np.array_equal(b.fflag.cpu().numpy()[sl], ff[sl].astype(np.int32))
+    if state in ("still", "creeping"):
+        assert np.array_equal(P, Po) and np.array_equal(U, Uo)
+    else:
+        assert np.array_equal(np.isfinite(P), np.isfinite(Po))
+        fin = np.isfinite(Po).all(axis=(1, 2, 3))
+        assert np.all(rel_err(P[fin], Po[fin]) <= RTOL) and np.all(rel_err(U[fin], Uo[fin]) <= RTOL)
