@@ -24,12 +24,22 @@ namespace khb {
 
 static constexpr double SMALL = 1e-20;          // decs.hpp:82
 
+// Resident 128-thread blocks per SM asked of the compiler for the face kernels
+#ifndef KHB_FLUX_EMHD_MINB
+#define KHB_FLUX_EMHD_MINB 3
+#endif
+
 enum { CL_CONSTANT = 0, CL_SOUNDSPEED = 1, CL_KAPPA_ETA = 2, CL_TORUS = 3 };
 enum { SOLVE_CONVERGED = 0, SOLVE_FAIL = 1, SOLVE_BEYOND_TOL = 2, SOLVE_BACKTRACK = 3 };
 
+// Threads per block of the Newton kernel: the Jacobians of a block (49 doubles a zone) fit static
+// shared memory, and four blocks an SM at 255 registers
+enum { IMP_BLOCK = 64 };
+
 // ------------------------------------------------------------------------------ closures
 // EMHD::set_parameters, scalar form (emhd.hpp:179-261); r is the zone-centre radius (torus closure)
-__device__ __forceinline__ void set_parameters(const EmhdArgs& E, double gam, double rho, double u, double qtilde,
+template <class AR>
+__device__ __forceinline__ void set_parameters(AR& ar, const EmhdArgs& E, double gam, double rho, double u, double qtilde,
                                                double dPtilde, double bsq, double r,
                                                double& tau, double& chi_e, double& nu_e)
 {
@@ -38,14 +48,15 @@ __device__ __forceinline__ void set_parameters(const EmhdArgs& E, double gam, do
         chi_e = E.conduction_alpha;
         nu_e = E.viscosity_alpha;
     } else if (E.closure == CL_SOUNDSPEED) {
-        const double cs2 = (gam * (gam - 1.) * u) / (rho + (gam * u));
+        const double cs2 = ar.div(gam * (gam - 1.) * u, rho + (gam * u));
         tau = E.tau;
         chi_e = E.conduction_alpha * cs2 * tau;
         nu_e = E.viscosity_alpha * cs2 * tau;
     } else if (E.closure == CL_KAPPA_ETA) {
         tau = E.tau;
-        chi_e = E.kappa / kmax(rho, SMALL);
-        nu_e = E.eta / kmax(rho, SMALL);
+        const auto rr = ar.rcp(kmax(rho, SMALL));
+        chi_e = ar.quot(E.kappa, rr);
+        nu_e = ar.quot(E.eta, rr);
     } else {
         const double tau_dyn = sqrt(r*r*r);
         tau = tau_dyn;
@@ -78,34 +89,38 @@ __device__ __forceinline__ void set_parameters(const EmhdArgs& E, double gam, do
 }
 
 // EMHD::convert_prims_to_q_dP (emhd.hpp:313-332)
-__device__ __forceinline__ void convert_q_dP(const EmhdArgs& E, double qt, double dPt, double rho, double Theta,
+template <class AR>
+__device__ __forceinline__ void convert_q_dP(AR& ar, const EmhdArgs& E, double qt, double dPt, double rho, double Theta,
                                              double cs2, double& q, double& dP)
 {
     q = qt;
     if (E.higher_order_terms) {
-        if (E.closure == CL_KAPPA_ETA) q *= sqrt(E.kappa * Theta * Theta / E.tau);
-        else                           q *= sqrt(rho * E.conduction_alpha * cs2 * Theta * Theta);
+        if (E.closure == CL_KAPPA_ETA) q *= ar.root(ar.div(E.kappa * Theta * Theta, E.tau));
+        else                           q *= ar.root(rho * E.conduction_alpha * cs2 * Theta * Theta);
     }
     dP = dPt;
     if (E.higher_order_terms) {
-        if (E.closure == CL_KAPPA_ETA) dP *= sqrt(E.eta * Theta / E.tau);
-        else                           dP *= sqrt(rho * E.viscosity_alpha * cs2 * Theta);
+        if (E.closure == CL_KAPPA_ETA) dP *= ar.root(ar.div(E.eta * Theta, E.tau));
+        else                           dP *= ar.root(rho * E.viscosity_alpha * cs2 * Theta);
     }
 }
 
 // Row T^dir_mu of the EMHD stress tensor (emhd.hpp:296-309) from the full q and dP
-__device__ __forceinline__ void emhd_tensor(double rho, double u, double pgas, double q, double dP,
+template <class AR>
+__device__ __forceinline__ void emhd_tensor(AR& ar, double rho, double u, double pgas, double q, double dP,
                                             const FourVec<double>& D, int dir, double T[4])
 {
     const double bsq = kmax(dot4(D.bcon, D.bcov), SMALL);
-    const double b_mag = sqrt(bsq);
+    const double b_mag = ar.root(bsq);
+    const double qb = ar.div(q, b_mag);
+    const auto rb = ar.rcp(bsq);
     const double eta = pgas + rho + u + bsq;
     const double ptot = pgas + 0.5 * bsq;
 #pragma unroll
     for (int mu = 0; mu < 4; ++mu)
         T[mu] = eta * D.ucon[dir] * D.ucov[mu] + ptot * (double)(dir == mu) - D.bcon[dir] * D.bcov[mu]
-              + (q / b_mag) * ((D.ucon[dir] * D.bcov[mu]) + (D.bcon[dir] * D.ucov[mu]))
-              - dP * ((D.bcon[dir] * D.bcov[mu] / bsq) - (1./3.) * ((double)(dir == mu) + D.ucon[dir] * D.ucov[mu]));
+              + qb * ((D.ucon[dir] * D.bcov[mu]) + (D.bcon[dir] * D.ucov[mu]))
+              - dP * (ar.quot(D.bcon[dir] * D.bcov[mu], rb) - (1./3.) * ((double)(dir == mu) + D.ucon[dir] * D.ucov[mu]));
 }
 
 // Zone-centre geometry for the EMHD kernels
@@ -129,6 +144,7 @@ __device__ __forceinline__ void load_center(const DevGeom& g, int j, int i, Cent
 __device__ __forceinline__ void emhd_p_to_u(const EmhdArgs& E, double gam, const CenterGeom& G, const double* P,
                                             double* U)
 {
+    Plain<double> ar;
     FourVec<double> D;
     calc_4vecs<double, true>(G.gcov, G.gcon0[0], G.gcon0, P, D);
     const double gdet = G.gdet;
@@ -136,11 +152,11 @@ __device__ __forceinline__ void emhd_p_to_u(const EmhdArgs& E, double gam, const
     double T[4];
     if ((E.conduction || E.viscosity) && E.feedback) {
         const double qt = E.conduction ? P[8] : 0., dPt = E.viscosity ? P[9] : 0.;
-        const double Theta = (gam - 1) * P[1] / P[0];
-        const double cs2 = gam * (gam - 1) * P[1] / (P[0] + gam * P[1]);
+        const double Theta = ar.div((gam - 1) * P[1], P[0]);
+        const double cs2 = ar.div(gam * (gam - 1) * P[1], P[0] + gam * P[1]);
         double q, dP;
-        convert_q_dP(E, qt, dPt, P[0], Theta, cs2, q, dP);
-        emhd_tensor(P[0], P[1], (gam - 1) * P[1], q, dP, D, 0, T);
+        convert_q_dP(ar, E, qt, dPt, P[0], Theta, cs2, q, dP);
+        emhd_tensor(ar, P[0], P[1], (gam - 1) * P[1], q, dP, D, 0, T);
     } else {
         calc_tensor<double, true>(P[0], P[1], (gam - 1) * P[1], D, 0, T);
     }
@@ -157,18 +173,19 @@ __device__ __forceinline__ void emhd_p_to_u(const EmhdArgs& E, double gam, const
 // Flux::prim_to_flux for the 10-slot state at any location (dir = 0: conserved variables), with the
 // EMHD stress tensor when q or dP feed back (flux_functions.hpp:80-107, 180-232).  Inactive EMHD
 // slots get 0.
-__device__ __forceinline__ void emhd_prim_to_flux(const EmhdArgs& E, double gam, double gdet, const double* P,
+template <class AR>
+__device__ __forceinline__ void emhd_prim_to_flux(AR& ar, const EmhdArgs& E, double gam, double gdet, const double* P,
                                                   const FourVec<double>& D, int dir, double* flux)
 {
     flux[0] = P[0] * D.ucon[dir] * gdet;
     double T[4];
     if ((E.conduction || E.viscosity) && E.feedback) {
         const double qt = E.conduction ? P[8] : 0., dPt = E.viscosity ? P[9] : 0.;
-        const double Theta = (gam - 1) * P[1] / P[0];
-        const double cs2 = gam * (gam - 1) * P[1] / (P[0] + gam * P[1]);
+        const double Theta = ar.div((gam - 1) * P[1], P[0]);
+        const double cs2 = ar.div(gam * (gam - 1) * P[1], P[0] + gam * P[1]);
         double q, dP;
-        convert_q_dP(E, qt, dPt, P[0], Theta, cs2, q, dP);
-        emhd_tensor(P[0], P[1], (gam - 1) * P[1], q, dP, D, dir, T);
+        convert_q_dP(ar, E, qt, dPt, P[0], Theta, cs2, q, dP);
+        emhd_tensor(ar, P[0], P[1], (gam - 1) * P[1], q, dP, D, dir, T);
     } else {
         calc_tensor<double, true>(P[0], P[1], (gam - 1) * P[1], D, dir, T);
     }
@@ -189,19 +206,20 @@ __device__ __forceinline__ void emhd_prim_to_flux(const EmhdArgs& E, double gam,
 
 // vchar with the EMHD-augmented sound speed (flux_functions.hpp:380-403); the closure parameters the
 // reference computes there are unused, so they are not formed
-__device__ __forceinline__ void emhd_vchar(const EmhdArgs& E, double gam, const double* P, const FourVec<double>& D,
+template <class AR>
+__device__ __forceinline__ void emhd_vchar(AR& ar, const EmhdArgs& E, double gam, const double* P, const FourVec<double>& D,
                                            double gcon00, double gcon0d, double gcondd, int dir,
                                            double& cmax, double& cmin)
 {
     const double ef  = P[0] + gam * P[1];
-    const double cs2 = gam * (gam - 1) * P[1] / ef;
+    const double cs2 = ar.div(gam * (gam - 1) * P[1], ef);
     const double bsq = dot4(D.bcon, D.bcov);
-    const double va2 = bsq / (bsq + ef);
+    const double va2 = ar.div(bsq, bsq + ef);
     const double ccond2 = E.conduction ? (gam - 1.) * E.conduction_alpha * cs2 : 0.0;
-    const double cvis2 = E.viscosity ? (4./3.) / (P[0] + (gam * P[1])) * P[0] * E.viscosity_alpha * cs2 : 0.0;
-    const double cs2_emhd = 0.5*(cs2 + ccond2 + sqrt(cs2*cs2 + ccond2*ccond2)) + cvis2;
+    const double cvis2 = E.viscosity ? ar.div(4./3., P[0] + (gam * P[1])) * P[0] * E.viscosity_alpha * cs2 : 0.0;
+    const double cs2_emhd = 0.5*(cs2 + ccond2 + ar.root(cs2*cs2 + ccond2*ccond2)) + cvis2;
     const double cms2 = cs2_emhd + va2 - cs2_emhd*va2;
-    vchar_speeds<double>(cms2, D, gcon00, gcon0d, gcondd, dir, cmax, cmin);
+    vchar_speeds<double>(ar, cms2, D, gcon00, gcon0d, gcondd, dir, cmax, cmin);
 }
 
 // ------------------------------------------------------------------------------ residual
@@ -246,8 +264,8 @@ struct Imp {
 
 // Set up the residual constants (calc_residual's sub-step-state and full-step-state parts,
 // implicit.hpp:161-198; emhd_sources.hpp:69-128).  Pf, Ps: 10-slot full-step and sub-step states.
-template <bool HQ, bool HD>
-__device__ __forceinline__ void setup_zone(const EmhdArgs& E, double gam, double r, const double* Pf, const double* Uf,
+template <bool HQ, bool HD, class AR>
+__device__ __forceinline__ void setup_zone(AR& ar, const EmhdArgs& E, double gam, double r, const double* Pf, const double* Uf,
                                            const double* Ps, const double* Sz, const double* Psol,
                                            ResidZone<Imp<HQ, HD>::NF>& Z)
 {
@@ -262,58 +280,60 @@ __device__ __forceinline__ void setup_zone(const EmhdArgs& E, double gam, double
     const CenterGeom& G = Z.G;
     // EMHD::set_parameters on the sub-step state (emhd.hpp:262-287)
     FourVec<double> Ds;
-    calc_4vecs<double, true>(G.gcov, G.gcon0[0], G.gcon0, Ps, Ds);
+    calc_4vecs<double, true>(ar, G.gcov, G.gcon0[0], G.gcon0, Ps, Ds);
     const double bsq = kmax(dot4(Ds.bcon, Ds.bcov), SMALL);
     const double qts = HQ ? Ps[8] : 0., dPts = HD ? Ps[9] : 0.;
-    set_parameters(E, gam, Ps[0], Ps[1], qts, dPts, bsq, r, Z.tau, Z.chi_e, Z.nu_e);
+    set_parameters(ar, E, gam, Ps[0], Ps[1], qts, dPts, bsq, r, Z.tau, Z.chi_e, Z.nu_e);
     const double tau = Z.tau, chi_e = Z.chi_e, nu_e = Z.nu_e;
     // time_derivative_sources constants
-    const double mag_b = sqrt(bsq);
+    const double mag_b = ar.root(bsq);
+    const auto rmb = ar.rcp(mag_b), rtau = ar.rcp(tau);
     {
         double ucon[4];
-        const double gamma = lorentz(G.gcov, Pf[2], Pf[3], Pf[4]);
-        const double alpha = 1. / sqrt(-G.gcon0[0]);
-        ucon[0] = gamma / alpha;
+        const double gamma = ar.root(lorentz_sq(G.gcov, Pf[2], Pf[3], Pf[4]));
+        const double alpha = ar.inv(ar.root(-G.gcon0[0]));
+        ucon[0] = ar.div(gamma, alpha);
 #pragma unroll
         for (int v = 0; v < 3; ++v) ucon[v+1] = Pf[2 + v] - gamma * alpha * G.gcon0[v+1];
         lower4(G.gcov, ucon, Z.ucov_old);
     }
-    Z.Theta_old = kmax((gam-1) * Pf[1] / Pf[0], SMALL);
+    Z.Theta_old = kmax(ar.div((gam-1) * Pf[1], Pf[0]), SMALL);
     const double rho = Ps[0];
-    const double Theta = (gam-1) * Ps[1] / Ps[0];
+    const double Theta = ar.div((gam-1) * Ps[1], Ps[0]);
     const double gdet = G.gdet;
     if (HQ) {
-        Z.cq0 = -rho * chi_e * (Ds.bcon[0] / mag_b);
+        Z.cq0 = -rho * chi_e * ar.quot(Ds.bcon[0], rmb);
 #pragma unroll
-        for (int mu = 0; mu < 4; ++mu) Z.cq[mu] = rho * chi_e * (Ds.bcon[mu] / mag_b) * Theta * Ds.ucon[0];
-        Z.fac_q = (chi_e != 0) ? sqrt(tau / (chi_e * rho * Theta * Theta)) : 0.0;
+        for (int mu = 0; mu < 4; ++mu) Z.cq[mu] = rho * chi_e * ar.quot(Ds.bcon[mu], rmb) * Theta * Ds.ucon[0];
+        Z.fac_q = (chi_e != 0) ? ar.root(ar.div(tau, chi_e * rho * Theta * Theta)) : 0.0;
         Z.gq = gdet * (qts / 2.);
-        Z.dUi_q = -gdet * (Pf[8] / tau);
-        Z.norm_q = (chi_e != 0) ? sqrt(rho * chi_e * tau * Theta * Theta) / tau : 1.;
+        Z.dUi_q = -gdet * ar.quot(Pf[8], rtau);
+        Z.norm_q = (chi_e != 0) ? ar.quot(ar.root(rho * chi_e * tau * Theta * Theta), rtau) : 1.;
     }
     if (HD) {
+        const auto rbsq = ar.rcp(bsq);
         Z.cd0 = -rho * nu_e;
 #pragma unroll
-        for (int mu = 0; mu < 4; ++mu) Z.cd[mu] = 3. * rho * nu_e * (Ds.bcon[0] * Ds.bcon[mu] / bsq);
-        Z.fac_d = (nu_e != 0) ? sqrt(tau / (nu_e * rho * Theta)) : 0.0;
+        for (int mu = 0; mu < 4; ++mu) Z.cd[mu] = 3. * rho * nu_e * ar.quot(Ds.bcon[0] * Ds.bcon[mu], rbsq);
+        Z.fac_d = (nu_e != 0) ? ar.root(ar.div(tau, nu_e * rho * Theta)) : 0.0;
         Z.gd = gdet * (dPts / 2.);
-        Z.dUi_d = -gdet * (Pf[9] / tau);
-        Z.norm_d = (nu_e != 0) ? sqrt(rho * nu_e * tau * Theta) / tau : 1.;
+        Z.dUi_d = -gdet * ar.quot(Pf[9], rtau);
+        Z.norm_d = (nu_e != 0) ? ar.quot(ar.root(rho * nu_e * tau * Theta), rtau) : 1.;
     }
 }
 
 // GRMHD::calc_4vecs of the trial state (grmhd_functions.hpp:225-246) and, for EMHD, the
 // time-derivative pieces of EMHD::time_derivative_sources (emhd_sources.hpp:84-93)
-template <bool HQ, bool HD>
-__device__ __forceinline__ void velocity_part(double dt, const ResidZone<Imp<HQ, HD>::NF>& Z, const double* x,
+template <bool HQ, bool HD, class AR>
+__device__ __forceinline__ void velocity_part(AR& ar, double dt, const ResidZone<Imp<HQ, HD>::NF>& Z, const double* x,
                                               VelState& V)
 {
     using I = Imp<HQ, HD>;
     const CenterGeom& G = Z.G;
     FourVec<double>& D = V.D;
-    V.gamma = lorentz(G.gcov, x[2], x[3], x[4]);
-    const double alpha = 1. / sqrt(-G.gcon0[0]);
-    D.ucon[0] = V.gamma / alpha;
+    V.gamma = ar.root(lorentz_sq(G.gcov, x[2], x[3], x[4]));
+    const double alpha = ar.inv(ar.root(-G.gcon0[0]));
+    D.ucon[0] = ar.div(V.gamma, alpha);
 #pragma unroll
     for (int v = 0; v < 3; ++v) D.ucon[v+1] = x[2 + v] - V.gamma * alpha * G.gcon0[v+1];
     lower4(G.gcov, D.ucon, D.ucov);
@@ -321,12 +341,13 @@ __device__ __forceinline__ void velocity_part(double dt, const ResidZone<Imp<HQ,
 #pragma unroll
     for (int v = 0; v < 3; ++v) b0 += Z.B[v] * D.ucov[v+1];
     D.bcon[0] = b0;
+    const auto ru0 = ar.rcp(D.ucon[0]), rdt = ar.rcp(dt);
 #pragma unroll
-    for (int v = 0; v < 3; ++v) D.bcon[v+1] = (Z.B[v] + b0 * D.ucon[v+1]) / D.ucon[0];
+    for (int v = 0; v < 3; ++v) D.bcon[v+1] = ar.quot(Z.B[v] + b0 * D.ucon[v+1], ru0);
     lower4(G.gcov, D.bcon, D.bcov);
     if (I::EM) {
 #pragma unroll
-        for (int mu = 0; mu < 4; ++mu) V.dt_ucov[mu] = (D.ucov[mu] - Z.ucov_old[mu]) / dt;
+        for (int mu = 0; mu < 4; ++mu) V.dt_ucov[mu] = ar.quot(D.ucov[mu] - Z.ucov_old[mu], rdt);
         double div_ucon = 0.;
 #pragma unroll
         for (int mu = 0; mu < 4; ++mu) div_ucon += G.gcon0[mu] * V.dt_ucov[mu];
@@ -336,8 +357,8 @@ __device__ __forceinline__ void velocity_part(double dt, const ResidZone<Imp<HQ,
 
 // Implicit::calc_residual (implicit.hpp:139-200) at the trial implicit variables x (rho, u, u1-u3[, q~][, dP~])
 // given their velocity part V
-template <bool HQ, bool HD>
-__device__ __forceinline__ void residual_with(const EmhdArgs& E, double gam, double dt,
+template <bool HQ, bool HD, class AR>
+__device__ __forceinline__ void residual_with(AR& ar, const EmhdArgs& E, double gam, double dt,
                                               const ResidZone<Imp<HQ, HD>::NF>& Z, const double* x,
                                               const VelState& V, double* res, ResidState& S)
 {
@@ -351,20 +372,22 @@ __device__ __forceinline__ void residual_with(const EmhdArgs& E, double gam, dou
     const double pgas = (gam - 1) * x[1];
     if (I::EM && E.feedback) {
         const double qt = HQ ? x[I::IQ] : 0., dPt = HD ? x[I::ID] : 0.;
-        S.Theta = (gam - 1) * x[1] / x[0];
-        S.cs2 = gam * (gam - 1) * x[1] / (x[0] + gam * x[1]);
-        convert_q_dP(E, qt, dPt, x[0], S.Theta, S.cs2, S.q, S.dP);
+        S.Theta = ar.div((gam - 1) * x[1], x[0]);
+        S.cs2 = ar.div(gam * (gam - 1) * x[1], x[0] + gam * x[1]);
+        convert_q_dP(ar, E, qt, dPt, x[0], S.Theta, S.cs2, S.q, S.dP);
         const double dot = dot4(D.bcon, D.bcov);
         S.bsq_clamped = dot < SMALL;
         S.bsq = kmax(dot, SMALL);
-        S.bmag = sqrt(S.bsq);
+        S.bmag = ar.root(S.bsq);
+        const double qb = ar.div(S.q, S.bmag);
+        const auto rb = ar.rcp(S.bsq);
         S.eta = pgas + x[0] + x[1] + S.bsq;
         const double ptot = pgas + 0.5 * S.bsq;
 #pragma unroll
         for (int mu = 0; mu < 4; ++mu)
             T[mu] = S.eta * D.ucon[0] * D.ucov[mu] + ptot * (double)(0 == mu) - D.bcon[0] * D.bcov[mu]
-                  + (S.q / S.bmag) * ((D.ucon[0] * D.bcov[mu]) + (D.bcon[0] * D.ucov[mu]))
-                  - S.dP * ((D.bcon[0] * D.bcov[mu] / S.bsq) - (1./3.) * ((double)(0 == mu) + D.ucon[0] * D.ucov[mu]));
+                  + qb * ((D.ucon[0] * D.bcov[mu]) + (D.bcon[0] * D.ucov[mu]))
+                  - S.dP * (ar.quot(D.bcon[0] * D.bcov[mu], rb) - (1./3.) * ((double)(0 == mu) + D.ucon[0] * D.ucov[mu]));
     } else {
         S.bsq = dot4(D.bcon, D.bcov);
         S.bsq_clamped = false;
@@ -377,24 +400,26 @@ __device__ __forceinline__ void residual_with(const EmhdArgs& E, double gam, dou
     U[4] = T[3] * gdet;
     if (HQ) U[I::IQ] = x[I::IQ] * D.ucon[0] * gdet;
     if (HD) U[I::ID] = x[I::ID] * D.ucon[0] * gdet;
+    const auto rdt = ar.rcp(dt);
 #pragma unroll
-    for (int p = 0; p < I::NF; ++p) res[p] = (U[p] - Z.Ui[p]) / dt - Z.S[p];
+    for (int p = 0; p < I::NF; ++p) res[p] = ar.quot(U[p] - Z.Ui[p], rdt) - Z.S[p];
     if (I::EM) {
         const double tau = Z.tau;
-        const double th = (gam-1) * x[1] / x[0];
+        const auto rtau = ar.rcp(tau);
+        const double th = ar.div((gam-1) * x[1], x[0]);
         S.theta_clamped = th < SMALL;
         const double Theta_new = kmax(th, SMALL);
-        const double dt_Theta = (Theta_new - Z.Theta_old) / dt;
+        const double dt_Theta = ar.quot(Theta_new - Z.Theta_old, rdt);
         if (HQ) {
             double rq = res[I::IQ];
-            const double dUq = -gdet * (x[I::IQ] / tau);
+            const double dUq = -gdet * ar.quot(x[I::IQ], rtau);
             rq -= 0.5*(dUq + Z.dUi_q);
             double q0 = Z.cq0 * dt_Theta;
 #pragma unroll
             for (int mu = 0; mu < 4; ++mu) q0 -= Z.cq[mu] * V.dt_ucov[mu];
             double q0t = q0;
             if (E.higher_order_terms) q0t *= Z.fac_q;
-            double dUqt = gdet * (q0t / tau);
+            double dUqt = gdet * ar.quot(q0t, rtau);
             if (E.higher_order_terms) dUqt += Z.gq * V.div_ucon;
             rq -= dUqt;
             rq *= tau;
@@ -403,14 +428,14 @@ __device__ __forceinline__ void residual_with(const EmhdArgs& E, double gam, dou
         }
         if (HD) {
             double rd = res[I::ID];
-            const double dUd = -gdet * (x[I::ID] / tau);
+            const double dUd = -gdet * ar.quot(x[I::ID], rtau);
             rd -= 0.5*(dUd + Z.dUi_d);
             double dP0 = Z.cd0 * V.div_ucon;
 #pragma unroll
             for (int mu = 0; mu < 4; ++mu) dP0 += Z.cd[mu] * V.dt_ucov[mu];
             double dP0t = dP0;
             if (E.higher_order_terms) dP0t *= Z.fac_d;
-            double dUdt_ = gdet * (dP0t / tau);
+            double dUdt_ = gdet * ar.quot(dP0t, rtau);
             if (E.higher_order_terms) dUdt_ += Z.gd * V.div_ucon;
             rd -= dUdt_;
             rd *= tau;
@@ -420,46 +445,50 @@ __device__ __forceinline__ void residual_with(const EmhdArgs& E, double gam, dou
     }
 }
 
-template <bool HQ, bool HD>
-__device__ __forceinline__ void residual(const EmhdArgs& E, double gam, double dt, const ResidZone<Imp<HQ, HD>::NF>& Z,
+template <bool HQ, bool HD, class AR>
+__device__ __forceinline__ void residual(AR& ar, const EmhdArgs& E, double gam, double dt, const ResidZone<Imp<HQ, HD>::NF>& Z,
                                          const double* x, double* res)
 {
     VelState V;
     ResidState S;
-    velocity_part<HQ, HD>(dt, Z, x, V);
-    residual_with<HQ, HD>(E, gam, dt, Z, x, V, res, S);
+    velocity_part<HQ, HD>(ar, dt, Z, x, V);
+    residual_with<HQ, HD>(ar, E, gam, dt, Z, x, V, res, S);
 }
 
 // Forward-difference Jacobian (Implicit::calc_jacobian, implicit.hpp:208-255).  res: residual at x.
-template <bool HQ, bool HD>
-__device__ __forceinline__ void jacobian_fd(const EmhdArgs& E, double gam, double dt, double delta,
+template <bool HQ, bool HD, class AR>
+__device__ __forceinline__ void jacobian_fd(AR& ar, const EmhdArgs& E, double gam, double dt, double delta,
                                             const ResidZone<Imp<HQ, HD>::NF>& Z, const double* x,
-                                            double* res, double (&J)[Imp<HQ, HD>::NF][Imp<HQ, HD>::NF])
+                                            double* res, double* Jm, long long js)
 {
     constexpr int NF = Imp<HQ, HD>::NF;
     VelState V0;
     ResidState S;
-    velocity_part<HQ, HD>(dt, Z, x, V0);
-    residual_with<HQ, HD>(E, gam, dt, Z, x, V0, res, S);
+    velocity_part<HQ, HD>(ar, dt, Z, x, V0);
+    residual_with<HQ, HD>(ar, E, gam, dt, Z, x, V0, res, S);
+    auto column = [&](int col, bool vel) {
+        double xc = x[0];
 #pragma unroll
-    for (int col = 0; col < NF; ++col) {
-        double xp[NF];
+        for (int p = 1; p < NF; ++p) xc = (p == col) ? x[p] : xc;
+        const double pert = (fabs(xc) < (0.5 * delta)) ? xc + delta : (1 + delta) * xc;
+        double xp[NF], rp[NF];
 #pragma unroll
-        for (int p = 0; p < NF; ++p) xp[p] = x[p];
-        if (fabs(x[col]) < (0.5 * delta)) xp[col] = x[col] + delta;
-        else xp[col] = (1 + delta) * x[col];
-        double rp[NF];
-        if (col >= 2 && col <= 4) {
+        for (int p = 0; p < NF; ++p) xp[p] = (p == col) ? pert : x[p];
+        if (vel) {
             VelState V;
-            velocity_part<HQ, HD>(dt, Z, xp, V);
-            residual_with<HQ, HD>(E, gam, dt, Z, xp, V, rp, S);
+            velocity_part<HQ, HD>(ar, dt, Z, xp, V);
+            residual_with<HQ, HD>(ar, E, gam, dt, Z, xp, V, rp, S);
         } else {
-            residual_with<HQ, HD>(E, gam, dt, Z, xp, V0, rp, S);
+            residual_with<HQ, HD>(ar, E, gam, dt, Z, xp, V0, rp, S);
         }
-        const double h = xp[col] - x[col] + SMALL;
+        const auto rh = ar.rcp(pert - xc + SMALL);
 #pragma unroll
-        for (int row = 0; row < NF; ++row) J[row][col] = (rp[row] - res[row]) / h;
-    }
+        for (int row = 0; row < NF; ++row) Jm[(row*NF + col)*js] = ar.quot(rp[row] - res[row], rh);
+    };
+#pragma unroll 1
+    for (int col = 2; col <= 4; ++col) column(col, true);
+#pragma unroll 1
+    for (int n = 0; n < NF - 3; ++n) column(n < 2 ? n : n + 3, false);
 }
 
 // Exact Jacobian of the same residual by a hand-written tangent.  Each column is one seed
@@ -470,31 +499,31 @@ __device__ __forceinline__ void jacobian_fd(const EmhdArgs& E, double gam, doubl
 // then the product rule through T^t_mu, the conserved variables and the EMHD source terms.  The
 // tangent is not bound to the reference's operation order, so divisions are replaced by products
 // with reciprocals computed once.
-template <bool HQ, bool HD>
-__device__ __forceinline__ void jacobian_exact(const EmhdArgs& E, double gam, double dt,
+template <bool HQ, bool HD, class AR>
+__device__ __forceinline__ void jacobian_exact(AR& ar, const EmhdArgs& E, double gam, double dt,
                                                const ResidZone<Imp<HQ, HD>::NF>& Z, const double* x,
-                                               double* res, double (&J)[Imp<HQ, HD>::NF][Imp<HQ, HD>::NF])
+                                               double* res, double* Jm, long long js)
 {
     using I = Imp<HQ, HD>;
     constexpr int NF = I::NF;
     VelState V;
     ResidState S;
-    velocity_part<HQ, HD>(dt, Z, x, V);
-    residual_with<HQ, HD>(E, gam, dt, Z, x, V, res, S);
+    velocity_part<HQ, HD>(ar, dt, Z, x, V);
+    residual_with<HQ, HD>(ar, E, gam, dt, Z, x, V, res, S);
     const CenterGeom& G = Z.G;
     const FourVec<double>& D = V.D;
     const double u0 = D.ucon[0], b0 = D.bcon[0];
     const double gdet = G.gdet, rho = x[0], uu = x[1];
-    const double inv_dt = 1. / dt, inv_u0 = 1. / u0, inv_rho = 1. / rho;
-    const double inv_tau = I::EM ? 1. / Z.tau : 0.;
+    const double inv_dt = ar.inv(dt), inv_u0 = ar.inv(u0), inv_rho = ar.inv(rho);
+    const double inv_tau = I::EM ? ar.inv(Z.tau) : 0.;
     const double gdt = gdet * inv_dt;
     const bool emt = I::EM && E.feedback;
     // EMHD tensor pieces: T^t_mu = ... + (q/|b|) X_mu - dP Y_mu
     double X[4], Y[4], qb = 0., fq = 1., fd = 1., inv_bsq = 0., inv_bmag = 0.;
     double dq[2] = {0., 0.}, ddP[2] = {0., 0.};
     if (emt) {
-        inv_bsq = 1. / S.bsq;
-        inv_bmag = 1. / S.bmag;
+        inv_bsq = ar.inv(S.bsq);
+        inv_bmag = ar.inv(S.bmag);
         qb = S.q * inv_bmag;
 #pragma unroll
         for (int mu = 0; mu < 4; ++mu) {
@@ -502,13 +531,13 @@ __device__ __forceinline__ void jacobian_exact(const EmhdArgs& E, double gam, do
             Y[mu] = b0 * D.bcov[mu] * inv_bsq - ((double)(mu == 0) + u0 * D.ucov[mu]) * (1. / 3.);
         }
         if (E.higher_order_terms) {
-            const double Th = S.Theta, cs2 = S.cs2, inv_den = 1. / (rho + gam * uu);
+            const double Th = S.Theta, cs2 = S.cs2, inv_den = ar.inv(rho + gam * uu);
             const double dTh[2] = {-Th * inv_rho, (gam - 1) * inv_rho};
             const double dcs2[2] = {-cs2 * inv_den, (gam * (gam - 1) - gam * cs2) * inv_den};
             const double qt = HQ ? x[I::IQ] : 0., dPt = HD ? x[I::ID] : 0.;
             double sq, sd, dsq[2], dsd[2];
             if (E.closure == CL_KAPPA_ETA) {
-                const double kt = E.kappa / E.tau, et = E.eta / E.tau;
+                const double kt = ar.div(E.kappa, E.tau), et = ar.div(E.eta, E.tau);
                 sq = kt * Th * Th;
                 sd = et * Th;
 #pragma unroll
@@ -544,7 +573,7 @@ __device__ __forceinline__ void jacobian_exact(const EmhdArgs& E, double gam, do
         if (HQ) dU[I::IQ] = (dqt * u0 + x[I::IQ] * du0) * gdt;
         if (HD) dU[I::ID] = (ddPt * u0 + x[I::ID] * du0) * gdt;
 #pragma unroll
-        for (int row = 0; row < NF; ++row) J[row][k] = dU[row];
+        for (int row = 0; row < 5; ++row) Jm[(row*NF + k)*js] = dU[row];
         if (HQ) {
             double dq0 = Z.cq0 * ddt_Theta;
             if (dtu) {
@@ -556,7 +585,7 @@ __device__ __forceinline__ void jacobian_exact(const EmhdArgs& E, double gam, do
             if (E.higher_order_terms) dsrc += Z.gq * ddiv;
             double dr = (dU[I::IQ] + 0.5 * gdet * dqt * inv_tau - dsrc) * Z.tau;
             if (E.higher_order_terms) dr *= Z.norm_q;
-            J[I::IQ][k] = dr;
+            Jm[(I::IQ*NF + k)*js] = dr;
         }
         if (HD) {
             double dd0 = Z.cd0 * ddiv;
@@ -569,7 +598,7 @@ __device__ __forceinline__ void jacobian_exact(const EmhdArgs& E, double gam, do
             if (E.higher_order_terms) dsrc += Z.gd * ddiv;
             double dr = (dU[I::ID] + 0.5 * gdet * ddPt * inv_tau - dsrc) * Z.tau;
             if (E.higher_order_terms) dr *= Z.norm_d;
-            J[I::ID][k] = dr;
+            Jm[(I::ID*NF + k)*js] = dr;
         }
     };
     const double dThn = (gam - 1) * inv_dt * inv_rho;
@@ -596,7 +625,7 @@ __device__ __forceinline__ void jacobian_exact(const EmhdArgs& E, double gam, do
         column(1, dT, 0., 0., 0., 0., S.theta_clamped ? 0. : dThn, 0., nullptr);
     }
     // velocities
-    const double inv_alpha = sqrt(-G.gcon0[0]), alpha = 1. / inv_alpha, inv_gamma = 1. / V.gamma;
+    const double inv_alpha = ar.root(-G.gcon0[0]), alpha = ar.inv(inv_alpha), inv_gamma = ar.inv(V.gamma);
 #pragma unroll
     for (int v = 0; v < 3; ++v) {
         double gk = 0.;
@@ -658,8 +687,8 @@ __device__ __forceinline__ void jacobian_exact(const EmhdArgs& E, double gam, do
 // operation order of KokkosBatched SerialQR / SerialApplyQ (left, transpose) / SerialTrsv (upper,
 // non-unit) / SerialApplyPivot (left, backward) as called at implicit.cpp:374-383.  Every index is
 // a compile-time constant so A stays in registers.
-template <int N>
-__device__ __forceinline__ void qr_solve(double (&A)[N][N], double (&b)[N])
+template <int N, class AR>
+__device__ __forceinline__ void qr_solve(AR& ar, double (&A)[N][N], double (&b)[N])
 {
     double tau[N], norm[N];
     int piv[N];
@@ -694,17 +723,17 @@ __device__ __forceinline__ void qr_solve(double (&A)[N][N], double (&b)[N])
         } else {
             const double chi1 = A[k][k];
             const double nchi1 = fabs(chi1);
-            const double nx = sqrt(nx2 + nchi1 * nchi1);
+            const double nx = ar.root(nx2 + nchi1 * nchi1);
             const double alph = (chi1 < 0 ? 1. : -1.) * nx;
             const double cma = chi1 - alph;
-            const double inv = 1. / cma;
+            const double inv = ar.inv(cma);
 #pragma unroll
             for (int r = k + 1; r < N; ++r) A[r][k] *= inv;
             const double cma2 = cma * cma;
-            tau[k] = 0.5 + 0.5 * (nx2 / cma2);
+            tau[k] = 0.5 + 0.5 * ar.div(nx2, cma2);
             A[k][k] = alph;
         }
-        const double inv_tau = 1. / tau[k];
+        const double inv_tau = ar.inv(tau[k]);
         double w[N];
 #pragma unroll
         for (int c = k + 1; c < N; ++c) {
@@ -724,7 +753,7 @@ __device__ __forceinline__ void qr_solve(double (&A)[N][N], double (&b)[N])
     }
 #pragma unroll
     for (int k = 0; k < N; ++k) {
-        const double inv_tau = 1. / tau[k];
+        const double inv_tau = ar.inv(tau[k]);
         double t = b[k];
 #pragma unroll
         for (int r = k + 1; r < N; ++r) t += A[r][k] * b[r];
@@ -735,7 +764,7 @@ __device__ __forceinline__ void qr_solve(double (&A)[N][N], double (&b)[N])
     }
 #pragma unroll
     for (int p = N - 1; p >= 0; --p) {
-        b[p] = b[p] / A[p][p];
+        b[p] = ar.div(b[p], A[p][p]);
 #pragma unroll
         for (int r = 0; r < p; ++r) b[r] -= A[r][p] * b[p];
     }
@@ -750,25 +779,25 @@ __device__ __forceinline__ void qr_solve(double (&A)[N][N], double (&b)[N])
 
 // The use_qr = false path: KokkosBatched SerialLU (no pivoting, diagonal nudged by SMALL) and the
 // upper-triangular solve alone, as implicit.cpp:387-401 calls them.
-template <int N>
-__device__ __forceinline__ void lu_solve(double (&A)[N][N], double (&b)[N])
+template <int N, class AR>
+__device__ __forceinline__ void lu_solve(AR& ar, double (&A)[N][N], double (&b)[N])
 {
 #pragma unroll
     for (int p = 0; p < N; ++p) {
         const double a_real = A[p][p];
         A[p][p] += -SMALL * (double)(a_real < 0);
         A[p][p] += SMALL * (double)(a_real >= 0);
-        const double a11 = A[p][p];
+        const auto a11 = ar.rcp(A[p][p]);
 #pragma unroll
         for (int r = p + 1; r < N; ++r) {
-            A[r][p] /= a11;
+            A[r][p] = ar.quot(A[r][p], a11);
 #pragma unroll
             for (int c = p + 1; c < N; ++c) A[r][c] -= A[r][p] * A[p][c];
         }
     }
 #pragma unroll
     for (int p = N - 1; p >= 0; --p) {
-        b[p] = b[p] / A[p][p];
+        b[p] = ar.div(b[p], A[p][p]);
 #pragma unroll
         for (int r = 0; r < p; ++r) b[r] -= A[r][p] * b[p];
     }
@@ -813,58 +842,85 @@ __global__ void __launch_bounds__(128) k_emhd_ptou(Dims d, DevGeom g, double gam
 // ------------------------------------------------------------------------------ explicit EMHD step
 // Flux::GetFlux with the EMHD variables (get_flux.hpp:60-373): one thread per face, every active
 // slot reconstructed, U and F with the EMHD tensor, EMHD signal speeds, LLF/HLLE.  F is [10][N].
-template <int DIR, int RECON, bool HQ, bool HD>
-__global__ void __launch_bounds__(128) k_flux_emhd(Dims d, DevGeom g, Phys ph, EmhdArgs E, khb_fields P,
-                                                   double* __restrict__ F, double* __restrict__ ctop, Box bx)
+// One face by the divisions and roots of policy AR; false where its operand checks failed
+template <int DIR, int RECON, bool HQ, bool HD, class AR>
+__device__ __forceinline__ bool flux_emhd_by(const Dims& d, const DevGeom& g, const Phys& ph, const EmhdArgs& E,
+                                             const khb_fields& P, double* __restrict__ F, double* __restrict__ ctop,
+                                             int i, int j, int k)
 {
-    int i, j, k;
-    if (!box_cell(bx, blockIdx.x, i, j, k)) return;
-    const long long c = ((long long)k*d.n2 + j)*d.n1 + i;
-    const long long st = (DIR == 1) ? 1 : ((DIR == 2) ? d.sj : d.sk);
+    AR ar;
+    const unsigned oc = (unsigned)(((long long)k*d.n2 + j)*d.n1 + i) * 8u;
+    const unsigned st = 8u * (unsigned)((DIR == 1) ? 1 : ((DIR == 2) ? d.sj : d.sk));
     const int loc = DIR - 1;
     const double gam = ph.gam;
-    const long long gi = (long long)j*g.G1 + i;
+    const unsigned gi = (unsigned)(j*g.G1 + i) * 8u;
     double gcov[4][4], gcon0[4];
 #pragma unroll
-    for (int m = 0; m < 16; ++m) gcov[m/4][m%4] = __ldg(g.gcov[loc] + m*g.gs + gi);
+    for (int m = 0; m < 16; ++m) gcov[m/4][m%4] = ldo(g.gcov[loc] + m*g.gs, gi);
 #pragma unroll
-    for (int m = 0; m < 4; ++m) gcon0[m] = __ldg(g.gcon[loc] + m*g.gs + gi);
-    const double gcondd = __ldg(g.gcon[loc] + (DIR*4 + DIR)*g.gs + gi);
-    const double gdet = __ldg(g.gdet[loc] + gi);
+    for (int m = 0; m < 4; ++m) gcon0[m] = ldo(g.gcon[loc] + m*g.gs, gi);
+    const double gcondd = ldo(g.gcon[loc] + (DIR*4 + DIR)*g.gs, gi);
+    const double gdet = ldo(g.gdet[loc], gi);
     double Pl[10], Pr[10];
 #pragma unroll
     for (int p = 0; p < 10; ++p) {
         const bool on = p < 8 || (p == 8 && HQ) || (p == 9 && HD);
         if (!on) { Pl[p] = Pr[p] = 0.; continue; }
         const double* q = P.v[p];
-        const double x0 = __ldg(q + c - 3*st), x1 = __ldg(q + c - 2*st), x2 = __ldg(q + c - st);
-        const double x3 = __ldg(q + c), x4 = __ldg(q + c + st), x5 = __ldg(q + c + 2*st);
-        Pl[p] = recon_right<RECON, double>(x0, x1, x2, x3, x4);
-        Pr[p] = recon_left<RECON, double>(x1, x2, x3, x4, x5);
+        const double x0 = ldo(q, oc - 3u*st), x1 = ldo(q, oc - 2u*st), x2 = ldo(q, oc - st);
+        const double x3 = ldo(q, oc), x4 = ldo(q, oc + st), x5 = ldo(q, oc + 2u*st);
+        if (RECON == RECON_WENO5) {
+            ar.bounded(x0); ar.bounded(x1); ar.bounded(x2); ar.bounded(x3); ar.bounded(x4); ar.bounded(x5);
+        }
+        Pl[p] = recon_right<RECON, double>(ar, x0, x1, x2, x3, x4);
+        Pr[p] = recon_left<RECON, double>(ar, x1, x2, x3, x4, x5);
     }
     FourVec<double> D;
     double Ul[10], Fl[10], Ur[10], Fr[10], cmaxL, cminL, cmaxR, cminR;
-    calc_4vecs<double, true>(gcov, gcon0[0], gcon0, Pl, D);
-    emhd_prim_to_flux(E, gam, gdet, Pl, D, 0, Ul);
-    emhd_prim_to_flux(E, gam, gdet, Pl, D, DIR, Fl);
-    emhd_vchar(E, gam, Pl, D, gcon0[0], gcon0[DIR], gcondd, DIR, cmaxL, cminL);
-    calc_4vecs<double, true>(gcov, gcon0[0], gcon0, Pr, D);
-    emhd_prim_to_flux(E, gam, gdet, Pr, D, 0, Ur);
-    emhd_prim_to_flux(E, gam, gdet, Pr, D, DIR, Fr);
-    emhd_vchar(E, gam, Pr, D, gcon0[0], gcon0[DIR], gcondd, DIR, cmaxR, cminR);
+    calc_4vecs<double, true>(ar, gcov, gcon0[0], gcon0, Pl, D);
+    emhd_prim_to_flux(ar, E, gam, gdet, Pl, D, 0, Ul);
+    emhd_prim_to_flux(ar, E, gam, gdet, Pl, D, DIR, Fl);
+    emhd_vchar(ar, E, gam, Pl, D, gcon0[0], gcon0[DIR], gcondd, DIR, cmaxL, cminL);
+    calc_4vecs<double, true>(ar, gcov, gcon0[0], gcon0, Pr, D);
+    emhd_prim_to_flux(ar, E, gam, gdet, Pr, D, 0, Ur);
+    emhd_prim_to_flux(ar, E, gam, gdet, Pr, D, DIR, Fr);
+    emhd_vchar(ar, E, gam, Pr, D, gcon0[0], gcon0[DIR], gcondd, DIR, cmaxR, cminR);
     const double cmax = kmax(kmax(0., cmaxL), cmaxR);
     const double cmin = -kmin(kmin(0., cminL), cminR);
+    const bool llf = ph.riemann == 0;
+    const auto rsum = ar.rcp(llf ? 1. : cmax + cmin);
 #pragma unroll
     for (int p = 0; p < 10; ++p) {
         const bool on = p < 8 || (p == 8 && HQ) || (p == 9 && HD);
         double f = 0.;
         if (on) {
-            if (ph.riemann == 0) f = 0.5 * (Fl[p] + Fr[p] - kmax(cmax, cmin) * (Ur[p] - Ul[p]));
-            else f = (cmax*Fl[p] + cmin*Fr[p] - cmax*cmin*(Ur[p] - Ul[p])) / (cmax + cmin);
+            if (llf) f = 0.5 * (Fl[p] + Fr[p] - kmax(cmax, cmin) * (Ur[p] - Ul[p]));
+            else f = ar.quot(cmax*Fl[p] + cmin*Fr[p] - cmax*cmin*(Ur[p] - Ul[p]), rsum);
         }
-        F[p*d.N + c] = f;
+        sto(F + p*d.N, oc, f);
     }
-    ctop[c] = kmax(cmax, cmin);
+    sto(ctop, oc, kmax(cmax, cmin));
+    // both sides' states run into these fluxes (a NaN anywhere makes them one)
+    ar.see(Fl[0] + Fr[0]); ar.see(Fl[1] + Fr[1]); ar.see(Ur[1] - Ul[1]);
+    return ar.ok();
+}
+template <int DIR, int RECON, bool HQ, bool HD>
+__device__ __noinline__ void flux_emhd_plain(const Dims& d, const DevGeom& g, const Phys& ph, const EmhdArgs& E,
+                                             const khb_fields& P, double* __restrict__ F, double* __restrict__ ctop,
+                                             int i, int j, int k)
+{
+    flux_emhd_by<DIR, RECON, HQ, HD, Plain<double>>(d, g, ph, E, P, F, ctop, i, j, k);
+}
+template <int DIR, int RECON, bool HQ, bool HD>
+__global__ void __launch_bounds__(128, KHB_FLUX_EMHD_MINB)
+k_flux_emhd(const __grid_constant__ Dims d, const __grid_constant__ DevGeom g, const __grid_constant__ Phys ph,
+            const __grid_constant__ EmhdArgs E, const __grid_constant__ khb_fields P, double* __restrict__ F,
+            double* __restrict__ ctop, Box bx)
+{
+    int i, j, k;
+    if (!box_cell(bx, blockIdx.x, i, j, k)) return;
+    if (!flux_emhd_by<DIR, RECON, HQ, HD, Exact64>(d, g, ph, E, P, F, ctop, i, j, k))
+        flux_emhd_plain<DIR, RECON, HQ, HD>(d, g, ph, E, P, F, ctop, i, j, k);
 }
 
 // dU/dt over the interior: -div F of every active slot (flux-CT for B), plus Flux::AddGeoSource with
@@ -916,8 +972,9 @@ __global__ void __launch_bounds__(128) k_emhd_dudt(Dims d, DevGeom g, Phys ph, E
                     const double Theta = (gam - 1) * Pz[1] / Pz[0];
                     const double cs2 = gam * (gam - 1) * Pz[1] / (Pz[0] + gam * Pz[1]);
                     double q, dP;
-                    convert_q_dP(E, qt, dPt, Pz[0], Theta, cs2, q, dP);
-                    emhd_tensor(Pz[0], Pz[1], (gam - 1) * Pz[1], q, dP, D, mu, Tmu);
+                    Plain<double> ar;
+                    convert_q_dP(ar, E, qt, dPt, Pz[0], Theta, cs2, q, dP);
+                    emhd_tensor(ar, Pz[0], Pz[1], (gam - 1) * Pz[1], q, dP, D, mu, Tmu);
                 } else {
                     calc_tensor<double, true>(Pz[0], Pz[1], (gam - 1) * Pz[1], D, mu, Tmu);
                 }
@@ -1028,7 +1085,8 @@ __global__ void __launch_bounds__(128) k_emhd_sources(Dims d, DevGeom g, const d
     calc_4vecs<double, true>(G.gcov, G.gcon0[0], G.gcon0, Pz, D);
     const double bsq = kmax(dot4(D.bcon, D.bcov), SMALL);
     double tau, chi_e, nu_e;
-    set_parameters(E, gam, Pz[0], Pz[1], E.conduction ? Pz[8] : 0., E.viscosity ? Pz[9] : 0., bsq,
+    Plain<double> ar;
+    set_parameters(ar, E, gam, Pz[0], Pz[1], E.conduction ? Pz[8] : 0., E.viscosity ? Pz[9] : 0., bsq,
                    g.rcen[(long long)j * d.n1 + i], tau, chi_e, nu_e);
     const long long N = d.N, sj = d.sj, sk = d.sk;
     const bool do_2d = d.ndim > 1, do_3d = d.ndim > 2;
@@ -1124,14 +1182,129 @@ __device__ __forceinline__ void block_max_norm(double v, unsigned long long* wor
     }
 }
 
-// One Newton iteration of Implicit::Step for every interior zone (implicit.cpp:286-522).
-// words[it-1]: maximum solve_norm of iteration it (bits); words[IMP_ITER_WORD]: iterations taken.
-template <bool HQ, bool HD, int JAC>
-__global__ void __launch_bounds__(128) k_implicit_iter(Dims d, DevGeom g, double gam, EmhdArgs E, ImplicitArgs ip,
-                                                       ImpFields f, double dt, unsigned long long* words, int iter)
+// The Newton iteration of one zone by the divisions and roots of policy AR: residual, Jacobian (through
+// the thread's column Jm of shared memory, so that its columns can be formed in a loop), solve, line
+// search, update.  False, with nothing written, where AR's operand checks failed.
+template <bool HQ, bool HD, int JAC, class AR>
+__device__ __forceinline__ bool newton_zone(const Dims& d, const DevGeom& g, double gam, const EmhdArgs& E,
+                                            const ImplicitArgs& ip, const ImpFields& f, double dt, int j, int i,
+                                            long long c, double* Jm, double& norm_out)
 {
     using I = Imp<HQ, HD>;
     constexpr int NF = I::NF;
+    AR ar;
+    double sf = f.solve_fail[c];
+    double sn = f.solve_norm[c];
+    if (sf != SOLVE_FAIL) {
+        sf = SOLVE_CONVERGED;
+        ResidZone<NF> Z;
+        load_center(g, j, i, Z.G);
+        double Pf[10], Uf[10], Ps[10], Sz[10], Psol[10];
+        load10(f.Pf, c, Pf); load10(f.Uf, c, Uf); load10(f.Ps, c, Ps); load10(f.S, c, Sz); load10(f.Psol, c, Psol);
+        setup_zone<HQ, HD>(ar, E, gam, g.rcen[(long long)j * d.n1 + i], Pf, Uf, Ps, Sz, Psol, Z);
+        double x[NF], xs[NF];
+#pragma unroll
+        for (int p = 0; p < 5; ++p) { x[p] = Psol[p]; xs[p] = Ps[p]; }
+        if (HQ) { x[I::IQ] = Psol[8]; xs[I::IQ] = Ps[8]; }
+        if (HD) { x[I::ID] = Psol[9]; xs[I::ID] = Ps[9]; }
+        double res[NF], delta[NF];
+        if (JAC == 1) jacobian_exact<HQ, HD>(ar, E, gam, dt, Z, x, res, Jm, IMP_BLOCK);
+        else jacobian_fd<HQ, HD>(ar, E, gam, dt, ip.jacobian_delta, Z, x, res, Jm, IMP_BLOCK);
+        double J[NF][NF];
+#pragma unroll
+        for (int p = 0; p < NF; ++p) {
+            delta[p] = -res[p];
+#pragma unroll
+            for (int q = 0; q < NF; ++q) J[p][q] = Jm[(p*NF + q)*IMP_BLOCK];
+        }
+        if (ip.use_qr) qr_solve<NF>(ar, J, delta);
+        else lu_solve<NF>(ar, J, delta);
+        // implicit_set_step (implicit.cpp:426-521)
+        bool failed_now = false;
+        double lambda = ip.linesearch_lambda;
+        if ((x[0] + lambda*delta[0] < 0.) || (x[1] + lambda*delta[1] < 0.)) {
+            sf = SOLVE_BACKTRACK;
+            lambda = 0.1;
+        }
+        if ((x[0] + lambda*delta[0] < 0.) || (x[1] + lambda*delta[1] < 0.)) {
+            sf = SOLVE_FAIL;
+#pragma unroll
+            for (int p = 0; p < NF; ++p) x[p] = xs[p];
+            failed_now = true;
+        }
+        if (!failed_now) {
+            if (ip.linesearch) {
+                double nrm = 0.;
+#pragma unroll
+                for (int p = 0; p < NF; ++p) nrm += res[p]*res[p];
+                sn = ar.root_or_zero(nrm);
+                const double f0 = 0.5 * sn;
+                const double fprime0 = -2. * f0;
+                for (int it = 0; it < ip.max_linesearch_iter; it++) {
+                    double xl[NF];
+#pragma unroll
+                    for (int p = 0; p < NF; ++p) xl[p] = x[p] + (lambda * delta[p]);
+                    residual<HQ, HD>(ar, E, gam, dt, Z, xl, res);
+                    nrm = 0.;
+#pragma unroll
+                    for (int p = 0; p < NF; ++p) nrm += res[p]*res[p];
+                    sn = ar.root_or_zero(nrm);
+                    const double f1 = 0.5 * sn;
+                    const int condition = f1 > (f0 * (1. - ip.linesearch_eps * lambda) + SMALL);
+                    const double denom = (f1 - f0 - (fprime0 * lambda)) * condition + (1 - condition);
+                    const double lambda_new = ar.div(-fprime0 * lambda * lambda, denom) * 0.5;
+                    lambda = lambda * (1 - condition) + (condition * lambda_new);
+                    if (condition == 0) break;
+                }
+            }
+#pragma unroll
+            for (int p = 0; p < NF; ++p) x[p] += lambda * delta[p];
+            residual<HQ, HD>(ar, E, gam, dt, Z, x, res);
+            double nrm = 0;
+#pragma unroll
+            for (int p = 0; p < NF; ++p) nrm += res[p]*res[p];
+            sn = ar.root_or_zero(nrm);
+            if (isnan(sn)) {
+                sf = SOLVE_FAIL;
+#pragma unroll
+                for (int p = 0; p < NF; ++p) x[p] = xs[p];
+            } else if (sn > ip.rootfind_tol) {
+                sf = SOLVE_BEYOND_TOL;
+            }
+        }
+        ar.see(sn);      // of the residual at the new state: everything before runs into it
+        if (!ar.ok()) return false;
+#pragma unroll
+        for (int p = 0; p < 5; ++p) f.Psol.v[p][c] = x[p];
+        if (HQ) f.Psol.v[8][c] = x[I::IQ];
+        if (HD) f.Psol.v[9][c] = x[I::ID];
+        f.solve_fail[c] = sf;
+        f.solve_norm[c] = sn;
+    }
+    norm_out = sn;
+    return true;
+}
+// The same zone with the operators themselves, out of line
+template <bool HQ, bool HD, int JAC>
+__device__ __noinline__ double newton_plain(const Dims& d, const DevGeom& g, double gam, const EmhdArgs& E,
+                                            const ImplicitArgs& ip, const ImpFields& f, double dt, int j, int i,
+                                            long long c, double* Jm)
+{
+    double sn = 0.;
+    newton_zone<HQ, HD, JAC, Plain<double>>(d, g, gam, E, ip, f, dt, j, i, c, Jm, sn);
+    return sn;
+}
+
+// One Newton iteration of Implicit::Step for every interior zone (implicit.cpp:286-522).
+// words[it-1]: maximum solve_norm of iteration it (bits); words[IMP_ITER_WORD]: iterations taken.
+template <bool HQ, bool HD, int JAC>
+__global__ void __launch_bounds__(IMP_BLOCK)
+k_implicit_iter(const __grid_constant__ Dims d, const __grid_constant__ DevGeom g, double gam,
+                const __grid_constant__ EmhdArgs E, const __grid_constant__ ImplicitArgs ip,
+                const __grid_constant__ ImpFields f, double dt, unsigned long long* words, int iter)
+{
+    constexpr int NF = Imp<HQ, HD>::NF;
+    __shared__ double sJ[NF*NF*IMP_BLOCK];
     if (iter > 1) {
         const double prev = __longlong_as_double((long long)words[iter - 2]);
         if ((iter - 1) >= ip.min_nonlinear_iter && prev < ip.rootfind_tol) return;   // the loop has ended
@@ -1141,87 +1314,10 @@ __global__ void __launch_bounds__(128) k_implicit_iter(Dims d, DevGeom g, double
     long long c;
     double norm_out = 0.;
     if (interior_zone(d, (long long)blockIdx.x * blockDim.x + threadIdx.x, k, j, i, c)) {
-        double sf = f.solve_fail[c];
-        double sn = f.solve_norm[c];
-        if (sf != SOLVE_FAIL) {
-            sf = SOLVE_CONVERGED;
-            ResidZone<NF> Z;
-            load_center(g, j, i, Z.G);
-            double Pf[10], Uf[10], Ps[10], Sz[10], Psol[10];
-            load10(f.Pf, c, Pf); load10(f.Uf, c, Uf); load10(f.Ps, c, Ps); load10(f.S, c, Sz); load10(f.Psol, c, Psol);
-            setup_zone<HQ, HD>(E, gam, g.rcen[(long long)j * d.n1 + i], Pf, Uf, Ps, Sz, Psol, Z);
-            double x[NF], xs[NF];
-#pragma unroll
-            for (int p = 0; p < 5; ++p) { x[p] = Psol[p]; xs[p] = Ps[p]; }
-            if (HQ) { x[I::IQ] = Psol[8]; xs[I::IQ] = Ps[8]; }
-            if (HD) { x[I::ID] = Psol[9]; xs[I::ID] = Ps[9]; }
-            double J[NF][NF], res[NF], delta[NF];
-            if (JAC == 1) jacobian_exact<HQ, HD>(E, gam, dt, Z, x, res, J);
-            else jacobian_fd<HQ, HD>(E, gam, dt, ip.jacobian_delta, Z, x, res, J);
-#pragma unroll
-            for (int p = 0; p < NF; ++p) delta[p] = -res[p];
-            if (ip.use_qr) qr_solve<NF>(J, delta);
-            else lu_solve<NF>(J, delta);
-            // implicit_set_step (implicit.cpp:426-521)
-            bool failed_now = false;
-            double lambda = ip.linesearch_lambda;
-            if ((x[0] + lambda*delta[0] < 0.) || (x[1] + lambda*delta[1] < 0.)) {
-                sf = SOLVE_BACKTRACK;
-                lambda = 0.1;
-            }
-            if ((x[0] + lambda*delta[0] < 0.) || (x[1] + lambda*delta[1] < 0.)) {
-                sf = SOLVE_FAIL;
-#pragma unroll
-                for (int p = 0; p < NF; ++p) x[p] = xs[p];
-                failed_now = true;
-            }
-            if (!failed_now) {
-                if (ip.linesearch) {
-                    double nrm = 0.;
-#pragma unroll
-                    for (int p = 0; p < NF; ++p) nrm += res[p]*res[p];
-                    sn = sqrt(nrm);
-                    const double f0 = 0.5 * sn;
-                    const double fprime0 = -2. * f0;
-                    for (int it = 0; it < ip.max_linesearch_iter; it++) {
-                        double xl[NF];
-#pragma unroll
-                        for (int p = 0; p < NF; ++p) xl[p] = x[p] + (lambda * delta[p]);
-                        residual<HQ, HD>(E, gam, dt, Z, xl, res);
-                        nrm = 0.;
-#pragma unroll
-                        for (int p = 0; p < NF; ++p) nrm += res[p]*res[p];
-                        sn = sqrt(nrm);
-                        const double f1 = 0.5 * sn;
-                        const int condition = f1 > (f0 * (1. - ip.linesearch_eps * lambda) + SMALL);
-                        const double denom = (f1 - f0 - (fprime0 * lambda)) * condition + (1 - condition);
-                        const double lambda_new = -fprime0 * lambda * lambda / denom * 0.5;
-                        lambda = lambda * (1 - condition) + (condition * lambda_new);
-                        if (condition == 0) break;
-                    }
-                }
-#pragma unroll
-                for (int p = 0; p < NF; ++p) x[p] += lambda * delta[p];
-                residual<HQ, HD>(E, gam, dt, Z, x, res);
-                double nrm = 0;
-#pragma unroll
-                for (int p = 0; p < NF; ++p) nrm += res[p]*res[p];
-                sn = sqrt(nrm);
-                if (isnan(sn)) {
-                    sf = SOLVE_FAIL;
-#pragma unroll
-                    for (int p = 0; p < NF; ++p) x[p] = xs[p];
-                } else if (sn > ip.rootfind_tol) {
-                    sf = SOLVE_BEYOND_TOL;
-                }
-            }
-#pragma unroll
-            for (int p = 0; p < 5; ++p) f.Psol.v[p][c] = x[p];
-            if (HQ) f.Psol.v[8][c] = x[I::IQ];
-            if (HD) f.Psol.v[9][c] = x[I::ID];
-            f.solve_fail[c] = sf;
-            f.solve_norm[c] = sn;
-        }
+        double* Jm = sJ + threadIdx.x;
+        double sn;
+        if (!newton_zone<HQ, HD, JAC, Exact64>(d, g, gam, E, ip, f, dt, j, i, c, Jm, sn))
+            sn = newton_plain<HQ, HD, JAC>(d, g, gam, E, ip, f, dt, j, i, c, Jm);
         norm_out = sn;
     }
     block_max_norm(norm_out, words + (iter - 1));
@@ -1241,21 +1337,18 @@ __global__ void __launch_bounds__(128) k_implicit_jacobian(Dims d, DevGeom g, do
     load_center(g, j, i, Z.G);
     double Pf[10], Uf[10], Ps[10], Sz[10], Psol[10];
     load10(f.Pf, c, Pf); load10(f.Uf, c, Uf); load10(f.Ps, c, Ps); load10(f.S, c, Sz); load10(f.Psol, c, Psol);
-    setup_zone<HQ, HD>(E, gam, g.rcen[(long long)j * d.n1 + i], Pf, Uf, Ps, Sz, Psol, Z);
+    Plain<double> ar;
+    setup_zone<HQ, HD>(ar, E, gam, g.rcen[(long long)j * d.n1 + i], Pf, Uf, Ps, Sz, Psol, Z);
     double x[NF];
 #pragma unroll
     for (int p = 0; p < 5; ++p) x[p] = Psol[p];
     if (HQ) x[I::IQ] = Psol[8];
     if (HD) x[I::ID] = Psol[9];
-    double J[NF][NF], res[NF];
-    if (JAC == 1) jacobian_exact<HQ, HD>(E, gam, dt, Z, x, res, J);
-    else jacobian_fd<HQ, HD>(E, gam, dt, ip.jacobian_delta, Z, x, res, J);
+    double res[NF];
+    if (JAC == 1) jacobian_exact<HQ, HD>(ar, E, gam, dt, Z, x, res, jac + c, d.N);
+    else jacobian_fd<HQ, HD>(ar, E, gam, dt, ip.jacobian_delta, Z, x, res, jac + c, d.N);
 #pragma unroll
-    for (int r = 0; r < NF; ++r) {
-        resid[r * d.N + c] = res[r];
-#pragma unroll
-        for (int q = 0; q < NF; ++q) jac[(r * NF + q) * d.N + c] = J[r][q];
-    }
+    for (int r = 0; r < NF; ++r) resid[r * d.N + c] = res[r];
 }
 
 // Implicit::FixSolve (fix_solve.cpp:44-130), pass 1: replacement values of failed zones from their
@@ -1330,9 +1423,9 @@ static void iter_hd(const Dims& d, const DevGeom& g, double gam, const EmhdArgs&
 {
     const long long nz = (long long)d.nx1 * d.nx2 * d.nx3;
     if (ip.jacobian == 1)
-        k_implicit_iter<HQ, HD, 1><<<blocks_for(nz, 128), 128, 0, st>>>(d, g, gam, E, ip, f, dt, words, iter);
+        k_implicit_iter<HQ, HD, 1><<<blocks_for(nz, IMP_BLOCK), IMP_BLOCK, 0, st>>>(d, g, gam, E, ip, f, dt, words, iter);
     else
-        k_implicit_iter<HQ, HD, 0><<<blocks_for(nz, 128), 128, 0, st>>>(d, g, gam, E, ip, f, dt, words, iter);
+        k_implicit_iter<HQ, HD, 0><<<blocks_for(nz, IMP_BLOCK), IMP_BLOCK, 0, st>>>(d, g, gam, E, ip, f, dt, words, iter);
 }
 template <bool HQ, bool HD>
 static void jac_hd(const Dims& d, const DevGeom& g, double gam, const EmhdArgs& E, const ImplicitArgs& ip,
@@ -1432,7 +1525,8 @@ __global__ void __launch_bounds__(128) k_emhd_limits(Dims d, DevGeom g, double g
     calc_4vecs<double, true>(G.gcov, G.gcon0[0], G.gcon0, Pz, D);
     const double bsq = kmax(dot4(D.bcon, D.bcov), SMALL);
     double q, dP;
-    convert_q_dP(E, qtilde, dPtilde, rho, Theta, cs*cs, q, dP);
+    Plain<double> ar;
+    convert_q_dP(ar, E, qtilde, dPtilde, rho, Theta, cs*cs, q, dP);
     int ef = 0;
     if (E.conduction) {
         const double qmax = 1.07 * rho * cs*cs*cs;
