@@ -1777,6 +1777,10 @@ static void zone_nv(const Dims& d, const DevGeom& g, const Phys& ph, const ZoneA
     case M_ZONE_CELL | M_KASTAUN: k_zone<NV, FT, M_ZONE_CELL | M_KASTAUN><<<nb, 128, 0, st>>>(d, g, ph, a, bx); break;
     case M_UTOP: k_zone<NV, FT, M_UTOP><<<nb, 128, 0, st>>>(d, g, ph, a, bx); break;
     case M_UTOP | M_KASTAUN: k_zone<NV, FT, M_UTOP | M_KASTAUN><<<nb, 128, 0, st>>>(d, g, ph, a, bx); break;
+    // B_CT blocks (8 variables)
+    case M_UPDATE | M_BCT: k_zone<NV, FT, (NV > 5) ? (M_UPDATE | M_BCT) : 0><<<nb, 128, 0, st>>>(d, g, ph, a, bx); break;
+    case M_ZONE_CELL | M_BCT: k_zone<NV, FT, (NV > 5) ? (M_ZONE_CELL | M_BCT) : 0><<<nb, 128, 0, st>>>(d, g, ph, a, bx); break;
+    case M_ZONE_CELL | M_BCT | M_KASTAUN: k_zone<NV, FT, (NV > 5) ? (M_ZONE_CELL | M_BCT | M_KASTAUN) : 0><<<nb, 128, 0, st>>>(d, g, ph, a, bx); break;
     case M_ZONE_FLOORS: k_zone<NV, FT, M_ZONE_FLOORS><<<nb, 128, 0, st>>>(d, g, ph, a, bx); break;
     default: k_zone<NV, FT, 0><<<nb, 128, 0, st>>>(d, g, ph, a, bx); break;
     }
