@@ -47,8 +47,12 @@ int check_fields(const khb_ctx* ctx, const khb_fields* f, const char* name)
 
 // ------------------------------------------------------------------ fluxes
 // k_lo <= k_hi: only the faces whose x3 index lies in [k_lo, k_hi]
-int launch_flux(khb_ctx* ctx, int dir, const khb_fields& P, cudaStream_t st, int k_lo = 0, int k_hi = -1)
+// reset_stage (1 or 2, with dir 1): the launch also resets what that stage's zone pass accumulates
+int launch_flux(khb_ctx* ctx, int dir, const khb_fields& P, cudaStream_t st, int k_lo = 0, int k_hi = -1,
+                int reset_stage = 0)
 {
+    int* const count = reset_stage ? ctx->fail_count : nullptr;
+    unsigned long long* const word = (reset_stage == 2) ? ctx->words : nullptr;
     const Dims& d = ctx->d;
     int lo[3], cnt[3];
     const int s[3] = {d.is, d.js, d.ks}, e[3] = {d.ie, d.je, d.ke};
@@ -67,10 +71,10 @@ int launch_flux(khb_ctx* ctx, int dir, const khb_fields& P, cudaStream_t st, int
     }
     if (ctx->fp32)
         Launch<float>::flux(ctx->cfg.recon, ctx->nv, dir, d, ctx->g, ctx->ph, P, (float*)ctx->F[dir-1],
-                            (float*)ctx->ctop[dir-1], lo, cnt, st);
+                            (float*)ctx->ctop[dir-1], lo, cnt, count, word, st);
     else
         Launch<double>::flux(ctx->cfg.recon, ctx->nv, dir, d, ctx->g, ctx->ph, P, (double*)ctx->F[dir-1],
-                             (double*)ctx->ctop[dir-1], lo, cnt, st);
+                             (double*)ctx->ctop[dir-1], lo, cnt, count, word, st);
     KHB_LAUNCHED(ctx);
     return KHB_OK;
 }
@@ -82,19 +86,14 @@ int launch_fix_flux_t(khb_ctx* ctx, const Phys& ph, cudaStream_t st, FT* F1 = nu
     // default: the context's flux arrays; the EMHD stage passes its 10-slot arrays (nv = 10)
     const Dims& d = ctx->d;
     if (!F1) { F1 = (FT*)ctx->F[0]; F2 = (FT*)ctx->F[1]; F3 = (FT*)ctx->F[2]; nv = ctx->nv; }
-    if (d.ndim >= 2 && (ph.zero_polar_flux || (nv > 5 && ph.fix_polar_flux))) {
-        for (int face = 2; face <= 3; ++face) {
-            if (!phys_face(d.bc[face])) continue;
-            Launch<FT>::fix_flux_x2(nv, d, ph, F1, F2, F3, face == 2, st);
-            KHB_LAUNCHED(ctx);
-        }
-    }
-    if (ph.check_inflow_in && phys_face(d.bc[0])) {
-        Launch<FT>::fix_flux_x1(d, F1, 1, st);
-        KHB_LAUNCHED(ctx);
-    }
-    if (ph.check_inflow_out && phys_face(d.bc[1])) {
-        Launch<FT>::fix_flux_x1(d, F1, 0, st);
+    int fixes = 0;
+    if (d.ndim >= 2 && (ph.zero_polar_flux || (nv > 5 && ph.fix_polar_flux)))
+        for (int face = 2; face <= 3; ++face)
+            if (phys_face(d.bc[face])) fixes |= 1 << (face - 2);
+    if (ph.check_inflow_in && phys_face(d.bc[0])) fixes |= 4;
+    if (ph.check_inflow_out && phys_face(d.bc[1])) fixes |= 8;
+    if (fixes) {
+        Launch<FT>::fix_flux(nv, d, ph, F1, F2, F3, fixes, st);
         KHB_LAUNCHED(ctx);
     }
     return KHB_OK;
@@ -231,21 +230,30 @@ int launch_boundaries(khb_ctx* ctx, const khb_fields& P, const khb_fields& U, cu
         if (rc) return rc;
     }
     // X1 faces over the interior j range, then X2 faces over all i, then the corner fix
-    for (int face = 0; face < 2; ++face) {
-        if (!phys_face(d.bc[face])) continue;
-        physical = true;
-        LaunchCommon::bc(nv, d, ctx->g, ctx->ph, P, U, face, xj ? 0 : d.js, xj ? d.n2 : d.je - d.js + 1, lo_k, cnt_k, st);
-        KHB_LAUNCHED(ctx);
-    }
-    if (d.ndim >= 2) {
-        for (int face = 2; face < 4; ++face) {
-            if (!phys_face(d.bc[face])) continue;
-            physical = true;
-            LaunchCommon::bc(nv, d, ctx->g, ctx->ph, P, U, face, 0, d.n1, lo_k, cnt_k, st);
+    // the two faces of a direction in one launch, unless one could read the other's ghost zones (a
+    // block thinner than its ghost layers)
+    auto faces = [&](int face, bool thick, int lo_a, int cnt_a, int lk, int ck) -> int {
+        const bool lo = phys_face(d.bc[face]), hi = phys_face(d.bc[face + 1]);
+        if (lo && hi && thick) {
+            LaunchCommon::bc(nv, d, ctx->g, ctx->ph, P, U, face, 2, lo_a, cnt_a, lk, ck, st);
+            KHB_LAUNCHED(ctx);
+            return KHB_OK;
+        }
+        for (int f = face; f < face + 2; ++f) {
+            if (!phys_face(d.bc[f])) continue;
+            LaunchCommon::bc(nv, d, ctx->g, ctx->ph, P, U, f, 1, lo_a, cnt_a, lk, ck, st);
             KHB_LAUNCHED(ctx);
         }
+        return KHB_OK;
+    };
+    int rc;
+    physical = phys_face(d.bc[0]) || phys_face(d.bc[1]);
+    if ((rc = faces(0, d.nx1 >= d.is, xj ? 0 : d.js, xj ? d.n2 : d.je - d.js + 1, lo_k, cnt_k))) return rc;
+    if (d.ndim >= 2) {
+        physical = physical || phys_face(d.bc[2]) || phys_face(d.bc[3]);
+        if ((rc = faces(2, d.nx2 >= d.js, 0, d.n1, lo_k, cnt_k))) return rc;
         if (ctx->cfg.fix_corner_inner && phys_face(d.bc[0]) && phys_face(d.bc[3])) {
-            LaunchCommon::bc(nv, d, ctx->g, ctx->ph, P, U, 0, 0, d.n2, lo_k, cnt_k, st);
+            LaunchCommon::bc(nv, d, ctx->g, ctx->ph, P, U, 0, 1, 0, d.n2, lo_k, cnt_k, st);
             KHB_LAUNCHED(ctx);
         }
     }
@@ -262,12 +270,9 @@ int launch_boundaries(khb_ctx* ctx, const khb_fields& P, const khb_fields& U, cu
     // the boundary planes with the X1/X2 ghost zones already filled; then B_P and U = U(P) there
     int kplanes = 0;
     if (d.ndim >= 3) {
-        for (int face = 4; face < 6; ++face) {
-            if (!phys_face(d.bc[face])) continue;
-            kplanes |= 1 << (face - 4);
-            LaunchCommon::bc(nv, d, ctx->g, ctx->ph, P, U, face, 0, d.n1 * d.n2, 0, 1, st);
-            KHB_LAUNCHED(ctx);
-        }
+        for (int face = 4; face < 6; ++face)
+            if (phys_face(d.bc[face])) kplanes |= 1 << (face - 4);
+        if ((rc = faces(4, d.nx3 >= d.ks, 0, d.n1 * d.n2, 0, 1))) return rc;
         if (kplanes) {
             LaunchCommon::ghost_ptou(nv_ptou, d, ctx->g, ctx->ph, P, U, st, Bf, ct_mask, kplanes, pfaces);
             KHB_LAUNCHED(ctx);
@@ -383,13 +388,16 @@ int launch_ghost_copy(khb_ctx* ctx, const khb_fields& Ps, const khb_fields& Us, 
 
 int zone_pass(khb_ctx* ctx, int stage, double dt, const khb_fields& Ps, const khb_fields& Us,
               const khb_fields& U0, const khb_fields& Pout, const khb_fields& Uout,
-              int32_t* pflag, int32_t* fflag, cudaStream_t st)
+              int32_t* pflag, int32_t* fflag, cudaStream_t st, bool reset = true)
 {
     const int s = stage - 1;
     // failed-zone counter, and on the last stage the timestep minimum (taken over bit patterns,
     // from the pattern of DBL_MAX), reset on the device so that the stage can be graph-captured
-    LaunchCommon::stage_reset(ctx->fail_count, stage == 2 ? ctx->words : nullptr, st);
-    KHB_LAUNCHED(ctx);
+    // (reset = false: the stage's x1 faces did it)
+    if (reset) {
+        LaunchCommon::stage_reset(ctx->fail_count, stage == 2 ? ctx->words : nullptr, st);
+        KHB_LAUNCHED(ctx);
+    }
     ZoneCall zc;
     zc.Ps = Ps; zc.Us = Us; zc.U0 = U0; zc.Pout = Pout; zc.Uout = Uout;
     zc.pflag = pflag; zc.fflag = fflag;
@@ -428,11 +436,11 @@ int do_stage(khb_ctx* ctx, int stage, double dt, const khb_fields& Ps, const khb
 {
     int rc;
     for (int dir = 1; dir <= ctx->d.ndim; ++dir)
-        if ((rc = launch_flux(ctx, dir, Ps, st))) return rc;
+        if ((rc = launch_flux(ctx, dir, Ps, st, 0, -1, dir == 1 ? stage : 0))) return rc;
     if ((rc = launch_fofc(ctx, stage, dt, Ps, Us, U0, st))) return rc;
     if ((rc = launch_fix_flux(ctx, ctx->ph, st))) return rc;
     if ((rc = launch_ghost_copy(ctx, Ps, Us, Pout, Uout, st))) return rc;
-    if ((rc = zone_pass(ctx, stage, dt, Ps, Us, U0, Pout, Uout, pflag, fflag, st))) return rc;
+    if ((rc = zone_pass(ctx, stage, dt, Ps, Us, U0, Pout, Uout, pflag, fflag, st, false))) return rc;
     if ((rc = launch_fixup(ctx, Pout, Uout, pflag, st))) return rc;
     return launch_boundaries(ctx, Pout, Uout, st);
 }

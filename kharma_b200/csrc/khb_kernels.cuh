@@ -328,8 +328,14 @@ __device__ __forceinline__ void flux_face(const Dims& d, const DevGeom& g, const
 template <int DIR, int RECON, int NV, typename R, typename FT>
 __global__ void __launch_bounds__(128, FluxMinBlocks<R, DIR>::value)
 k_flux(const __grid_constant__ Dims d, const __grid_constant__ DevGeom g, const __grid_constant__ Phys ph,
-       const __grid_constant__ khb_fields P, FT* __restrict__ F, FT* __restrict__ ctop, Box bx)
+       const __grid_constant__ khb_fields P, FT* __restrict__ F, FT* __restrict__ ctop, Box bx, int* fail_count,
+       unsigned long long* word)
 {
+    // the stage's first launch also resets the failed-zone counter and the timestep minimum
+    if (DIR == 1 && fail_count && blockIdx.x == 0 && threadIdx.x == 0) {
+        *fail_count = 0;
+        if (word) *word = 0x7FEFFFFFFFFFFFFFull;             // bit pattern of DBL_MAX
+    }
     int i, j, k;
     if (!box_cell(bx, blockIdx.x, i, j, k)) return;
     flux_face<DIR, RECON, NV, R, FT>(d, g, ph, P, F, ctop, i, j, k);
@@ -364,11 +370,6 @@ __device__ __forceinline__ void fix_x2_zone(const Dims& d, const Phys& ph, FT* F
 #pragma unroll
         for (int p = 0; p < NV; ++p) F2[p*N + c] = (FT)0;
 }
-template <int NV, typename FT>
-__global__ void k_fix_flux_x2(Dims d, Phys ph, FT* F1, FT* F2, FT* F3, int inner)
-{
-    fix_x2_zone<NV, FT>(d, ph, F1, F2, F3, inner, blockIdx.x * blockDim.x + threadIdx.x);
-}
 template <typename FT>
 __device__ __forceinline__ void fix_x1_zone(const Dims& d, FT* F1, int inner, int t)
 {
@@ -382,10 +383,16 @@ __device__ __forceinline__ void fix_x1_zone(const Dims& d, FT* F1, int inner, in
     FT& f = F1[c];
     f = inner ? kmin(f, (FT)0) : kmax(f, (FT)0);
 }
-template <typename FT>
-__global__ void k_fix_flux_x1(Dims d, FT* F1, int inner)
+// The flux fixes of one block in one launch: blockIdx.y picks the n-th fix of `fixes` (bits 0, 1: inner
+// and outer x2 face; 2, 3: inner and outer x1 face); they touch disjoint faces and slots
+template <int NV, typename FT>
+__global__ void __launch_bounds__(128) k_fix_flux(Dims d, Phys ph, FT* F1, FT* F2, FT* F3, int fixes)
 {
-    fix_x1_zone<FT>(d, F1, inner, blockIdx.x * blockDim.x + threadIdx.x);
+    int f = __ffs(fixes) - 1;
+    for (unsigned n = 0; n < blockIdx.y; ++n) { fixes &= fixes - 1; f = __ffs(fixes) - 1; }
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (f >= 2) fix_x1_zone<FT>(d, F1, f == 2, t);
+    else fix_x2_zone<NV, FT>(d, ph, F1, F2, F3, f == 0, t);
 }
 // The flux fixes of every block of a batch in one launch: blockIdx.y picks a block's fix (its faces
 // and slots are disjoint from every other fix's)
@@ -1060,7 +1067,7 @@ template <int NV>
 __global__ void k_bc(Dims d, DevGeom g, Phys ph, khb_fields P, khb_fields U, int face,
                      int lo_a, int cnt_a, int lo_k, int cnt_k)
 {
-    bc_zone<NV>(d, g, ph, P, U, face, lo_a, cnt_a, lo_k, cnt_k, (long long)blockIdx.x * blockDim.x + threadIdx.x);
+    bc_zone<NV>(d, g, ph, P, U, face + (int)blockIdx.y, lo_a, cnt_a, lo_k, cnt_k, (long long)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 // Ghost zones of one (j, i) plane, enumerated without the interior: the rows below js, the zones
@@ -1702,49 +1709,53 @@ __global__ void k_batch_reset(int* const* counts, int nblocks, unsigned long lon
 // ===================================================================================== launchers
 template <int DIR, int NV, typename FT>
 static void flux_dir_recon(int recon, const Dims& d, const DevGeom& g, const Phys& ph, const khb_fields& P,
-                           FT* F, FT* ctop, const int lo[3], const int cnt[3], cudaStream_t st)
+                           FT* F, FT* ctop, const int lo[3], const int cnt[3], int* fail_count,
+                           unsigned long long* word, cudaStream_t st)
 {
     const Box bx = make_box(lo[0], lo[1], lo[2], cnt[0], cnt[1], cnt[2]);
     const unsigned nb = box_blocks(bx);
     switch (recon) {
-    case RECON_DONOR: k_flux<DIR, RECON_DONOR, NV, FT, FT><<<nb, 128, 0, st>>>(d, g, ph, P, F, ctop, bx); break;
-    case RECON_MC:    k_flux<DIR, RECON_MC, NV, FT, FT><<<nb, 128, 0, st>>>(d, g, ph, P, F, ctop, bx); break;
-    case RECON_WENO5: k_flux<DIR, RECON_WENO5, NV, FT, FT><<<nb, 128, 0, st>>>(d, g, ph, P, F, ctop, bx); break;
-    case RECON_PPM:   k_flux<DIR, RECON_PPM, NV, FT, FT><<<nb, 128, 0, st>>>(d, g, ph, P, F, ctop, bx); break;
-    case RECON_WENO5X: k_flux<DIR, RECON_WENO5X, NV, FT, FT><<<nb, 128, 0, st>>>(d, g, ph, P, F, ctop, bx); break;
-    default:          k_flux<DIR, RECON_EXTRA, NV, FT, FT><<<nb, 128, 0, st>>>(d, g, ph, P, F, ctop, bx); break;
+    case RECON_DONOR: k_flux<DIR, RECON_DONOR, NV, FT, FT><<<nb, 128, 0, st>>>(d, g, ph, P, F, ctop, bx, fail_count, word); break;
+    case RECON_MC:    k_flux<DIR, RECON_MC, NV, FT, FT><<<nb, 128, 0, st>>>(d, g, ph, P, F, ctop, bx, fail_count, word); break;
+    case RECON_WENO5: k_flux<DIR, RECON_WENO5, NV, FT, FT><<<nb, 128, 0, st>>>(d, g, ph, P, F, ctop, bx, fail_count, word); break;
+    case RECON_PPM:   k_flux<DIR, RECON_PPM, NV, FT, FT><<<nb, 128, 0, st>>>(d, g, ph, P, F, ctop, bx, fail_count, word); break;
+    case RECON_WENO5X: k_flux<DIR, RECON_WENO5X, NV, FT, FT><<<nb, 128, 0, st>>>(d, g, ph, P, F, ctop, bx, fail_count, word); break;
+    default:          k_flux<DIR, RECON_EXTRA, NV, FT, FT><<<nb, 128, 0, st>>>(d, g, ph, P, F, ctop, bx, fail_count, word); break;
     }
 }
 
 template <int NV, typename FT>
 static void flux_nv(int recon, int dir, const Dims& d, const DevGeom& g, const Phys& ph, const khb_fields& P,
-                    FT* F, FT* ctop, const int lo[3], const int cnt[3], cudaStream_t st)
+                    FT* F, FT* ctop, const int lo[3], const int cnt[3], int* fail_count,
+                           unsigned long long* word, cudaStream_t st)
 {
-    if (dir == 1) flux_dir_recon<1, NV, FT>(recon, d, g, ph, P, F, ctop, lo, cnt, st);
-    else if (dir == 2) flux_dir_recon<2, NV, FT>(recon, d, g, ph, P, F, ctop, lo, cnt, st);
-    else flux_dir_recon<3, NV, FT>(recon, d, g, ph, P, F, ctop, lo, cnt, st);
+    if (dir == 1) flux_dir_recon<1, NV, FT>(recon, d, g, ph, P, F, ctop, lo, cnt, fail_count, word, st);
+    else if (dir == 2) flux_dir_recon<2, NV, FT>(recon, d, g, ph, P, F, ctop, lo, cnt, fail_count, word, st);
+    else flux_dir_recon<3, NV, FT>(recon, d, g, ph, P, F, ctop, lo, cnt, fail_count, word, st);
 }
 
 template <typename FT>
 void Launch<FT>::flux(int recon, int nv, int dir, const Dims& d, const DevGeom& g, const Phys& ph,
-                      const khb_fields& P, FT* F, FT* ctop, const int lo[3], const int cnt[3], cudaStream_t st)
+                      const khb_fields& P, FT* F, FT* ctop, const int lo[3], const int cnt[3], int* fail_count,
+                           unsigned long long* word, cudaStream_t st)
 {
     // the kernel variant: KHB_RECON_* 0-3 as they are, 4-7 through RECON_EXTRA, WENO5 with lowering
     // or the floor fallback through RECON_WENO5X
     const int kr = (recon > RECON_PPM) ? RECON_EXTRA
                  : ((recon == RECON_WENO5 && (ph.weno_lower || ph.recon_fallback)) ? RECON_WENO5X : recon);
-    if (nv == 8) flux_nv<8, FT>(kr, dir, d, g, ph, P, F, ctop, lo, cnt, st);
-    else flux_nv<5, FT>(kr, dir, d, g, ph, P, F, ctop, lo, cnt, st);
+    if (nv == 8) flux_nv<8, FT>(kr, dir, d, g, ph, P, F, ctop, lo, cnt, fail_count, word, st);
+    else flux_nv<5, FT>(kr, dir, d, g, ph, P, F, ctop, lo, cnt, fail_count, word, st);
 }
 
 template <typename FT>
-void Launch<FT>::fix_flux_x2(int nv, const Dims& d, const Phys& ph, FT* F1, FT* F2, FT* F3, int inner, cudaStream_t st)
+void Launch<FT>::fix_flux(int nv, const Dims& d, const Phys& ph, FT* F1, FT* F2, FT* F3, int fixes, cudaStream_t st)
 {
-    const int ni = d.ie - d.is + 3, nk = (d.ndim > 2) ? d.ke - d.ks + 3 : 1;
-    const unsigned nb = blocks_for((long long)ni*nk, 128);
-    if (nv == 10) k_fix_flux_x2<10, FT><<<nb, 128, 0, st>>>(d, ph, F1, F2, F3, inner);
-    else if (nv == 8) k_fix_flux_x2<8, FT><<<nb, 128, 0, st>>>(d, ph, F1, F2, F3, inner);
-    else k_fix_flux_x2<5, FT><<<nb, 128, 0, st>>>(d, ph, F1, F2, F3, inner);
+    const int ni = d.ie - d.is + 3, nj = (d.ndim > 1) ? d.je - d.js + 3 : 1, nk = (d.ndim > 2) ? d.ke - d.ks + 3 : 1;
+    const int across = (fixes & 3) ? ((fixes & 12) ? max(ni, nj) : ni) : nj;
+    const dim3 grid(blocks_for((long long)across*nk, 128), (unsigned)__builtin_popcount((unsigned)fixes));
+    if (nv == 10) k_fix_flux<10, FT><<<grid, 128, 0, st>>>(d, ph, F1, F2, F3, fixes);
+    else if (nv == 8) k_fix_flux<8, FT><<<grid, 128, 0, st>>>(d, ph, F1, F2, F3, fixes);
+    else k_fix_flux<5, FT><<<grid, 128, 0, st>>>(d, ph, F1, F2, F3, fixes);
 }
 
 template <typename FT>
@@ -1754,13 +1765,6 @@ void Launch<FT>::fix_tasks(int nv, const FixTask<FT>* tasks, int ntasks, int max
     const dim3 grid(blocks_for(max_count, 128), (unsigned)ntasks);
     if (nv == 8) k_fix_tasks<8, FT><<<grid, 128, 0, st>>>(tasks);
     else k_fix_tasks<5, FT><<<grid, 128, 0, st>>>(tasks);
-}
-
-template <typename FT>
-void Launch<FT>::fix_flux_x1(const Dims& d, FT* F1, int inner, cudaStream_t st)
-{
-    const int nj = (d.ndim > 1) ? d.je - d.js + 3 : 1, nk = (d.ndim > 2) ? d.ke - d.ks + 3 : 1;
-    k_fix_flux_x1<FT><<<blocks_for((long long)nj*nk, 128), 128, 0, st>>>(d, F1, inner);
 }
 
 template <int NV, typename FT>
@@ -2041,10 +2045,10 @@ void LaunchCommon::fixup(int nv, const Dims& d, const DevGeom& g, const Phys& ph
 }
 
 void LaunchCommon::bc(int nv, const Dims& d, const DevGeom& g, const Phys& ph, const khb_fields& P, const khb_fields& U,
-                      int face, int lo_a, int cnt_a, int lo_k, int cnt_k, cudaStream_t st)
+                      int face, int nfaces, int lo_a, int cnt_a, int lo_k, int cnt_k, cudaStream_t st)
 {
     const int ng = (face < 2) ? d.is : ((face < 4) ? d.js : d.ks);
-    const unsigned nb = blocks_for((long long)ng*cnt_a*cnt_k, 128);
+    const dim3 nb(blocks_for((long long)ng*cnt_a*cnt_k, 128), (unsigned)nfaces);
     if (nv == 10) k_bc<10><<<nb, 128, 0, st>>>(d, g, ph, P, U, face, lo_a, cnt_a, lo_k, cnt_k);
     else if (nv == 8) k_bc<8><<<nb, 128, 0, st>>>(d, g, ph, P, U, face, lo_a, cnt_a, lo_k, cnt_k);
     else k_bc<5><<<nb, 128, 0, st>>>(d, g, ph, P, U, face, lo_a, cnt_a, lo_k, cnt_k);

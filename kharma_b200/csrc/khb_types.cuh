@@ -210,10 +210,12 @@ struct FixupBlock {
 // reference's rounding); Launch<float> (the FP32-flux form) is compiled with contraction.
 template <typename FT>
 struct Launch {
+    // fail_count (x1 faces only, may be NULL): reset here for the stage, and word when given
     static void flux(int recon, int nv, int dir, const Dims& d, const DevGeom& g, const Phys& ph,
-                     const khb_fields& P, FT* F, FT* ctop, const int lo[3], const int cnt[3], cudaStream_t st);
-    static void fix_flux_x2(int nv, const Dims& d, const Phys& ph, FT* F1, FT* F2, FT* F3, int inner, cudaStream_t st);
-    static void fix_flux_x1(const Dims& d, FT* F1, int inner, cudaStream_t st);
+                     const khb_fields& P, FT* F, FT* ctop, const int lo[3], const int cnt[3], int* fail_count,
+                     unsigned long long* word, cudaStream_t st);
+    // fixes: bits 0, 1 the inner and outer polar x2 face, 2, 3 the inner and outer x1 inflow check
+    static void fix_flux(int nv, const Dims& d, const Phys& ph, FT* F1, FT* F2, FT* F3, int fixes, cudaStream_t st);
     // the flux fixes of many blocks in one launch (max_count: the largest task's zone count)
     static void fix_tasks(int nv, const FixTask<FT>* tasks, int ntasks, int max_count, cudaStream_t st);
     static void zone(int nv, const Dims& d, const DevGeom& g, const Phys& ph, const ZoneArgs<FT>& a, cudaStream_t st);
@@ -249,8 +251,9 @@ struct Launch {
 struct LaunchCommon {
     static void fixup(int nv, const Dims& d, const DevGeom& g, const Phys& ph, const khb_fields& P, const khb_fields& U,
                       const int32_t* pflag, const int* fail_count, const int* fail_list, cudaStream_t st);
+    // nfaces = 2: the outer face of the direction (face + 1) in the same launch
     static void bc(int nv, const Dims& d, const DevGeom& g, const Phys& ph, const khb_fields& P, const khb_fields& U,
-                   int face, int lo_a, int cnt_a, int lo_k, int cnt_k, cudaStream_t st);
+                   int face, int nfaces, int lo_a, int cnt_a, int lo_k, int cnt_k, cudaStream_t st);
     // kplanes: the ghost planes of physical X3 faces (bit 0: below ks, bit 1: above ke) instead of
     // the X1/X2 ghost zones of the interior planes.  pfaces (nonzero): only the zones past the faces
     // whose bits are set (bit f: face f = inner/outer X1, X2, X3), the boundary domains of a block
