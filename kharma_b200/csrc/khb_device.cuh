@@ -437,7 +437,8 @@ __device__ __forceinline__ void vchar_speeds(AR& ar, R cms2, const FourVec<R>& D
     const R A  = Bu*Bu - (Bsq + Bu*Bu) * cms2;
     const R Bq = R(2.) * (Au*Bu - (AB + Au*Bu) * cms2);
     const R Cq = Au*Au - (Asq + Au*Au) * cms2;
-    const R discr = ar.root(kmax(Bq * Bq - R(4.) * A * Cq, R(0)));
+    // zero where a reconstruction overshot into a negative pressure
+    const R discr = ar.root_or_zero(kmax(Bq * Bq - R(4.) * A * Cq, R(0)));
     const auto r2A = ar.rcp(R(2.) * A);
     const R vp = ar.quot(-(-Bq + discr), r2A);
     const R vm = ar.quot(-(-Bq - discr), r2A);
@@ -634,17 +635,23 @@ __device__ __forceinline__ int u_to_p_onedw(AR& ar, const ZoneGeom& G, double ga
     Wp += dW;
     err = residual(Wp);
     int iter = 0;
+    // one exit, so that the lanes of a warp meet again behind the loop
+    bool run = max_iterations > 0;
 #pragma unroll 1
-    for (iter = 0; iter < max_iterations; iter++) {
+    while (run) {
         dW = ar.div((Wp1 - Wp) * err, err - err1);
         ar.see(dW);
         dW = kclip(dW, -0.5*Wp, 2.0*Wp);
         Wp1 = Wp;
         err1 = err;
         Wp += dW;
-        if (FAST ? fabs(dW) < tol * fabs(Wp) : ratio_below(dW, Wp, tol)) break;
-        err = residual(Wp);
-        if (FAST ? fabs(err) < tol * fabs(Wp) : ratio_below(err, Wp, tol)) break;
+        bool stop = FAST ? fabs(dW) < tol * fabs(Wp) : ratio_below(dW, Wp, tol);
+        if (!stop) {
+            err = residual(Wp);
+            stop = FAST ? fabs(err) < tol * fabs(Wp) : ratio_below(err, Wp, tol);
+        }
+        if (!stop) ++iter;
+        run = !stop && iter < max_iterations;
     }
     if (iter == max_iterations) return ST_MAX_ITER;
     const double W = Wp + D;
@@ -769,14 +776,24 @@ struct KastaunResidual {
         int iterations = max_iterations;
         if ((fabs(zm - zp) < tol) || ((fabs(fm) + fabs(fp)) < 2.0 * tol)) iterations = -1;
         double z = 0.5 * (zm + zp);
+        // one exit, so that the lanes of a warp meet again behind the loop
+        iter = 0;
+        bool run = iterations > 0;
 #pragma unroll 1
-        for (iter = 0; iter < iterations; ++iter) {
+        while (run) {
             z = ar.div(zm * fp - zp * fm, fp - fm);
             ar.see(z);
             const double fz = MASTER ? master(z) : aux(z);
-            if ((fabs(zm - zp) < tol) || (fabs(fz) < tol)) break;
-            if (fz * fp < 0.0) { zm = zp; fm = fp; zp = z; fp = fz; }
-            else { fm = 0.5 * fm; zp = z; fp = fz; }
+            const bool stop = (fabs(zm - zp) < tol) || (fabs(fz) < tol);
+            if (!stop) {
+                const bool cross = fz * fp < 0.0;
+                zm = cross ? zp : zm;
+                fm = cross ? fp : 0.5 * fm;
+                zp = z;
+                fp = fz;
+                ++iter;
+            }
+            run = !stop && iter < iterations;
         }
         return z;
     }
