@@ -511,17 +511,15 @@ __device__ __forceinline__ void ct_zone_b_edge(const Dims& d, const DevGeom& g, 
 
 // The geometric source of one zone (flux.cpp:413-441): new_du[lam] = sum over mu, nu of
 // T^mu_nu gdet Gamma^nu_lam mu for the UU and U1-U3 components, from the zone's primitives Ps
-template <int NV, class AR>
-__device__ __forceinline__ void geo_source(AR& ar, const Dims& d, const DevGeom& g, const ZoneGeom& G, double gam,
-                                           const double* Ps, int j, int i, double new_du[4])
+// conn(m): entry m = (nu*4 + lam)*4 + mu of the table
+template <int NV, class AR, class CONN>
+__device__ __forceinline__ void geo_source_with(AR& ar, const double gcov[4][4], const double* gcon0, double gam,
+                                                const double* Ps, CONN conn, double new_du[4])
 {
     FourVec<double> D;
-    const double gcon0[4] = {G.gcon[0][0], G.gcon[0][1], G.gcon[0][2], G.gcon[0][3]};
-    calc_4vecs<double, (NV > 5)>(ar, G.gcov, G.gcon[0][0], gcon0, Ps, D);
+    calc_4vecs<double, (NV > 5)>(ar, gcov, gcon0[0], gcon0, Ps, D);
 #pragma unroll
     for (int lam = 0; lam < 4; ++lam) new_du[lam] = 0.;
-    const unsigned cg = (unsigned)(j*g.n1 + i) * 8u;
-    const long long cs = (long long)(d.n2)*g.n1;
 #pragma unroll
     for (int mu = 0; mu < 4; ++mu) {
         double Tmu[4];
@@ -530,8 +528,17 @@ __device__ __forceinline__ void geo_source(AR& ar, const Dims& d, const DevGeom&
         for (int nu = 0; nu < 4; ++nu)
 #pragma unroll
             for (int lam = 0; lam < 4; ++lam)
-                new_du[lam] += Tmu[nu] * ldo(g.gdet_conn + ((nu*4 + lam)*4 + mu)*cs, cg);
+                new_du[lam] += Tmu[nu] * conn((nu*4 + lam)*4 + mu);
     }
+}
+template <int NV, class AR>
+__device__ __forceinline__ void geo_source(AR& ar, const Dims& d, const DevGeom& g, const ZoneGeom& G, double gam,
+                                           const double* Ps, int j, int i, double new_du[4])
+{
+    const double gcon0[4] = {G.gcon[0][0], G.gcon[0][1], G.gcon[0][2], G.gcon[0][3]};
+    const unsigned cg = (unsigned)(j*g.n1 + i) * 8u;
+    const long long cs = (long long)(d.n2)*g.n1;
+    geo_source_with<NV>(ar, G.gcov, gcon0, gam, Ps, [&](int m) { return ldo(g.gdet_conn + m*cs, cg); }, new_du);
 }
 
 // MODE: compile-time mask of M_* steps (0: take the mask from the arguments at run time).  The
@@ -761,6 +768,146 @@ k_zone(const __grid_constant__ Dims d, const __grid_constant__ DevGeom g, const 
     double ndt_zone = 1.7976931348623157e308;
     if (box_cell(bx, blockIdx.x, i, j, k)) ndt_zone = zone_body<NV, FT, MODE>(d, g, ph, a, i, j, k);
     if (a.mode & M_DT) block_min_ndt(ndt_zone, a.ndt_word);
+}
+
+// ------------------------------------------------------------------ update half, 3D blocks
+// The update half of a 3D block by columns: a warp takes 32 neighbouring (j, i) positions and steps through
+// `run` consecutive planes of them, four warps of a block through four runs.
+// What bounds it is the latency and the addresses of its loads: a zone reads 84 entries of the x3-independent
+// geometry (metric, connection), 30 face fluxes, 48 B fluxes for its 12 corner EMFs and 24 state values.  The
+// block stages the geometry of its positions in shared memory once for all its planes, at offsets that
+// are constants of the instruction, and the upper x3 faces and the EMFs above a zone are kept for the next
+// one (8 EMFs and 5 x3 fluxes a zone instead of 12 and 10).  Same operations in the same order as zone_by.
+enum { UPD_GCOV = 0, UPD_GCON0 = 16, UPD_CONN = 20, UPD_ENTRIES = 84 };
+#ifndef KHB_UPDATE3_MINB
+#define KHB_UPDATE3_MINB 3
+#endif
+template <int NV, typename FT>
+__global__ void __launch_bounds__(128, KHB_UPDATE3_MINB)
+k_update3(const __grid_constant__ Dims d, const __grid_constant__ DevGeom g, const __grid_constant__ Phys ph,
+          const __grid_constant__ ZoneArgs<FT> a, unsigned tiles, int run)
+{
+    __shared__ double sg[UPD_ENTRIES][32];
+    const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const unsigned bk = blockIdx.x / tiles, tile = blockIdx.x - bk * tiles;
+    const unsigned p = tile * 32u + lane, np = (unsigned)d.nx1 * (unsigned)d.nx2;
+    const bool in = p < np;
+    const unsigned pj = (in ? p : 0u) / (unsigned)d.nx1;
+    const int i = d.is + (int)((in ? p : 0u) - pj * (unsigned)d.nx1), j = d.js + (int)pj;
+    if (!ph.cart_minkowski) {
+        // entry e of the tables by warp e mod 4 (a row of 32 positions at a time)
+        const unsigned gi = (unsigned)kchk(d, (long long)j*g.G1 + i, g.gs, CHK_GEOM) * 8u, cg = (unsigned)(j*g.n1 + i) * 8u;
+        const long long cs = (long long)d.n2*g.n1;
+        for (int e = (int)warp; e < UPD_ENTRIES; e += 4) {
+            double x;
+            if (e < UPD_GCON0) {
+                // the FP32-flux form reads the upper triangle (load_zone_geom)
+                const int r = e / 4, q = e % 4;
+                x = ldo(g.gcov[3] + ((sizeof(FT) == 4 && q < r) ? q*4 + r : e)*g.gs, gi);
+            } else if (e < UPD_CONN) {
+                x = ldo(g.gcon[3] + (e - UPD_GCON0)*g.gs, gi);
+            } else {
+                x = ldo(g.gdet_conn + (e - UPD_CONN)*cs, cg);
+            }
+            sg[e][lane] = x;
+        }
+        __syncthreads();
+    }
+    const int k0 = d.ks + ((int)bk * 4 + (int)warp) * run;
+    int planes = d.ke + 1 - k0;
+    if (planes > run) planes = run;
+    if (!in || planes <= 0) return;
+
+    constexpr int NH = 5;
+    constexpr unsigned s1 = sizeof(FT);
+    const long long N = d.N;
+    const FT* F1 = a.F[0]; const FT* F2 = a.F[1]; const FT* F3 = a.F[2];
+    const unsigned sj = (unsigned)d.sj * s1, sk = (unsigned)d.sk * s1;
+    const double a1 = ph.dx2*ph.dx3, a2 = ph.dx1*ph.dx3, a3 = ph.dx1*ph.dx2;
+    const double bdt = a.dt_dev ? a.beta * __ldg(a.dt_dev) : a.bdt;
+    const bool lo_pole = ph.zero_polar_flux && j == d.js && phys_face(d.bc[2]);
+    const bool hi_pole = ph.zero_polar_flux && j == d.je && phys_face(d.bc[3]);
+    auto at = [&](const FT* F, unsigned x) -> FT {
+        return ldo(F, KHB_BOUNDS_CHECK ? (unsigned)kchk(d, x / s1, N, CHK_ZONE_CT) * s1 : x);
+    };
+    const FT* F1B2 = F1 + 6*N; const FT* F1B3 = F1 + 7*N; const FT* F2B1 = F2 + 5*N; const FT* F2B3 = F2 + 7*N;
+    const FT* F3B1 = F3 + 5*N; const FT* F3B2 = F3 + 6*N;
+    auto e3 = [&](unsigned x) -> FT { return (FT)0.25 * (at(F1B2, x) + at(F1B2, x - sj) - at(F2B1, x) - at(F2B1, x - s1)); };
+    auto e1 = [&](unsigned x) -> FT { return (FT)0.25 * (at(F2B3, x) + at(F2B3, x - sk) - at(F3B2, x) - at(F3B2, x - sj)); };
+    auto e2 = [&](unsigned x) -> FT { return (FT)0.25 * (at(F3B1, x) + at(F3B1, x - s1) - at(F1B3, x) - at(F1B3, x - sk)); };
+
+    long long c = kchk(d, ((long long)k0*d.n2 + j)*d.n1 + i, N, CHK_ZONE_FLUX);
+    FT f3[NH], e1a = 0, e1b = 0, e2a = 0, e2b = 0;      // x3 fluxes and EMFs below the zone
+    {
+        const unsigned of = (unsigned)c * s1;
+#pragma unroll
+        for (int q = 0; q < NH; ++q) f3[q] = ldo(F3 + q*N, of);
+        if (NV > 5) { e1a = e1(of); e1b = e1(of + sj); e2a = e2(of); e2b = e2(of + s1); }
+    }
+#pragma unroll 1
+    for (int n = 0; n < planes; ++n, c += d.sk) {
+        kchk(d, c + d.sk, N, CHK_ZONE_FLUX);
+        Exact64 ar;
+        const auto rvol = ar.rcp(ph.dx1*ph.dx2*ph.dx3);
+        const unsigned of = (unsigned)c * s1, oc = (unsigned)c * 8u;
+        double dudt[NV];
+#pragma unroll
+        for (int q = 0; q < NH; ++q) {
+            const FT up = ldo(F3 + q*N, of + sk);
+            double du = (a1 * ldfo(F1 + q*N, of + s1) - a1 * ldfo(F1 + q*N, of));
+            du += a2 * ldfo(F2 + q*N, of + sj) - a2 * ldfo(F2 + q*N, of);
+            du += a3 * (double)up - a3 * (double)f3[q];
+            f3[q] = up;
+            dudt[q] = ar.quot(-du, rvol);
+        }
+        if (NV > 5) {
+            // flux-CT as ct_divergence forms it: face fluxes from the EMFs, then their differences
+            const FT c00 = e3(of), c01 = e3(of + sj), c10 = e3(of + s1), c11 = e3(of + s1 + sj);
+            const FT u1a = e1(of + sk), u1b = e1(of + sj + sk), u2a = e2(of + sk), u2b = e2(of + s1 + sk);
+            const double f12lo = (double)((FT)0.5 * (c00 + c01)), f12hi = (double)((FT)0.5 * (c10 + c11));
+            const double f13lo = (double)((FT)-0.5 * (e2a + u2a)), f13hi = (double)((FT)-0.5 * (e2b + u2b));
+            const double f21lo = lo_pole ? 0. : (double)((FT)-0.5 * (c00 + c10));
+            const double f21hi = hi_pole ? 0. : (double)((FT)-0.5 * (c01 + c11));
+            const double f23lo = lo_pole ? 0. : (double)((FT)0.5 * (e1a + u1a));
+            const double f23hi = hi_pole ? 0. : (double)((FT)0.5 * (e1b + u1b));
+            const double f31lo = (double)((FT)0.5 * (e2a + e2b)), f31hi = (double)((FT)0.5 * (u2a + u2b));
+            const double f32lo = (double)((FT)-0.5 * (e1a + e1b)), f32hi = (double)((FT)-0.5 * (u1a + u1b));
+            e1a = u1a; e1b = u1b; e2a = u2a; e2b = u2b;
+            double du;
+            du = (a1 * 0. - a1 * 0.); du += a2 * f21hi - a2 * f21lo; du += a3 * f31hi - a3 * f31lo;
+            dudt[5] = ar.quot(-du, rvol);
+            du = (a1 * f12hi - a1 * f12lo); du += a2 * 0. - a2 * 0.; du += a3 * f32hi - a3 * f32lo;
+            dudt[6] = ar.quot(-du, rvol);
+            du = (a1 * f13hi - a1 * f13lo); du += a2 * f23hi - a2 * f23lo; du += a3 * 0. - a3 * 0.;
+            dudt[7] = ar.quot(-du, rvol);
+        }
+        if (!ph.cart_minkowski) {
+            double Ps[NV], gcov[4][4], gcon0[4], new_du[4];
+#pragma unroll
+            for (int q = 0; q < NV; ++q) Ps[q] = ldo(a.Ps.v[q], oc);
+#pragma unroll
+            for (int m = 0; m < 16; ++m) gcov[m/4][m%4] = sg[UPD_GCOV + m][lane];
+#pragma unroll
+            for (int m = 0; m < 4; ++m) gcon0[m] = sg[UPD_GCON0 + m][lane];
+            geo_source_with<NV>(ar, gcov, gcon0, ph.gam, Ps, [&](int m) { return sg[UPD_CONN + m][lane]; }, new_du);
+#pragma unroll
+            for (int v = 0; v < 4; ++v) dudt[1 + v] += new_du[v];
+        }
+        double U[NV];
+#pragma unroll
+        for (int q = 0; q < NV; ++q) {
+            const double x = a.g0 * ldo(a.Us.v[q], oc) + a.g1 * ldo(a.U0.v[q], oc);
+            U[q] = 1.0 * x + bdt * dudt[q];
+        }
+        ar.see(U[1]);
+        if (NV > 5) { ar.see(U[5]); ar.see(U[6]); ar.see(U[7]); }
+        if (ar.ok()) {
+#pragma unroll
+            for (int q = 0; q < NV; ++q) sto(a.Uout.v[q], oc, U[q]);
+        } else {
+            zone_plain<NV, FT, M_UPDATE>(d, g, ph, a, i, j, k0 + n);
+        }
+    }
 }
 
 // ===================================================================================== FOFC
@@ -1767,9 +1914,30 @@ void Launch<FT>::fix_tasks(int nv, const FixTask<FT>* tasks, int ntasks, int max
     else k_fix_tasks<5, FT><<<grid, 128, 0, st>>>(tasks);
 }
 
+// Planes a warp of k_update3 steps through: as many as leave four blocks an SM and slot to start with, at
+// most 8 (128^3 torus: 8 planes; the geometry is then read once for 32 planes)
+static int update3_run(unsigned tiles, int nk)
+{
+    for (int run = 8; run > 1; run /= 2)
+        if (tiles * (unsigned)((nk + 4*run - 1) / (4*run)) >= 4u * 148u * KHB_UPDATE3_MINB) return run;
+    return 1;
+}
+template <int NV, typename FT>
+static void update3(const Dims& d, const DevGeom& g, const Phys& ph, const ZoneArgs<FT>& a, cudaStream_t st)
+{
+    const unsigned tiles = ((unsigned)d.nx1 * (unsigned)d.nx2 + 31u) / 32u;
+    const int run = update3_run(tiles, d.nx3);
+    k_update3<NV, FT><<<tiles * (unsigned)((d.nx3 + 4*run - 1) / (4*run)), 128, 0, st>>>(d, g, ph, a, tiles, run);
+}
+
 template <int NV, typename FT>
 static void zone_nv(const Dims& d, const DevGeom& g, const Phys& ph, const ZoneArgs<FT>& a, cudaStream_t st)
 {
+    // the update half of a 3D block runs by columns (B_CT blocks, which read no EMFs there, lose 3% by it)
+    if (d.ndim == 3 && a.mode == M_UPDATE) {
+        update3<NV, FT>(d, g, ph, a, st);
+        return;
+    }
     const Box bx = make_box(d.is, d.js, d.ks, d.ie - d.is + 1, d.je - d.js + 1, d.ke - d.ks + 1);
     const unsigned nb = box_blocks(bx);
     const int m = a.mode & ~M_DT;
