@@ -33,7 +33,10 @@ enum { CL_CONSTANT = 0, CL_SOUNDSPEED = 1, CL_KAPPA_ETA = 2, CL_TORUS = 3 };
 enum { SOLVE_CONVERGED = 0, SOLVE_FAIL = 1, SOLVE_BEYOND_TOL = 2, SOLVE_BACKTRACK = 3 };
 
 // Threads per block of the Newton kernel: the Jacobians of a block (49 doubles a zone) fit static
-// shared memory, and four blocks an SM at 255 registers
+// shared memory, and four blocks an SM at 255 registers (5 or 6 blocks spill: 1730 against 1530 us for the
+// forward-difference solve at 128 x 96 x 64).  What bounds it is the length of one zone's chain of FP64
+// operations at 8 warps an SM (25% issue); before the branch-free arithmetic and the column loops it was
+// instruction fetch (64 x 64 x 48, one iteration: 426 to 218 us; exact Jacobian 182 to 129 us)
 enum { IMP_BLOCK = 64 };
 
 // ------------------------------------------------------------------------------ closures

@@ -181,8 +181,8 @@ __device__ __forceinline__ void prefetch_o(const T* base, unsigned off) { prefet
 // values written are then to be replaced).
 // What bounds a FP64 face is instruction issue and the FP64 pipe: with the compiler's divisions and 64-bit
 // addresses a linear-MC face took 3420 warp instructions, a third of them FP64, at 64% issue; with
-// Exact64 and 32-bit offsets 1660, 59% of them FP64, at 57% issue and 66% of the FP64 pipe (96^3 torus:
-// 152 to 85 us along x1, 173 to 84 along x3).
+// Exact64 and 32-bit offsets 1590, 61% of them FP64, at 59% issue and 71% of the FP64 pipe (96^3 torus:
+// 152 to 79 us along x1, 173 to 79 along x3).
 template <int DIR, int RECON, int NV, typename R, typename FT, class AR>
 __device__ __forceinline__ bool flux_face_by(const Dims& d, const DevGeom& g, const Phys& ph, const khb_fields& P,
                                           FT* __restrict__ F, FT* __restrict__ ctop, int i, int j, int k)
@@ -733,7 +733,7 @@ template <int NV, typename FT, int MODE>
 __device__ __forceinline__ double zone_body(const Dims& d, const DevGeom& g, const Phys& ph, const ZoneArgs<FT>& a,
                                             int i, int j, int k)
 {
-    if (!zone_by<NV, FT, MODE, Exact64>(d, g, ph, a, i, j, k)) zone_plain<NV, FT, MODE>(d, g, ph, a, i, j, k);
+    if (!zone_by<NV, FT, MODE, typename ZoneArith<FT>::type>(d, g, ph, a, i, j, k)) zone_plain<NV, FT, MODE>(d, g, ph, a, i, j, k);
     if (!(a.mode & M_DT)) return 1.7976931348623157e308;
     // grmhd.cpp:313-328
     const long long c = kchk(d, ((long long)k*d.n2 + j)*d.n1 + i, d.N, CHK_ZONE_FLUX);
@@ -778,6 +778,9 @@ k_zone(const __grid_constant__ Dims d, const __grid_constant__ DevGeom g, const 
 // block stages the geometry of its positions in shared memory once for all its planes, at offsets that
 // are constants of the instruction, and the upper x3 faces and the EMFs above a zone are kept for the next
 // one (8 EMFs and 5 x3 fluxes a zone instead of 12 and 10).  Same operations in the same order as zone_by.
+// 128^3 torus: 337 us as one zone per thread, 254 so (96^3: 188 to 137 us, 2.5 TB/s of DRAM); 168 registers
+// and 3 blocks an SM measured the same as 128 and 4, 2 blocks 2% slower; an L2 prefetch of the next plane
+// cost 3%.
 enum { UPD_GCOV = 0, UPD_GCON0 = 16, UPD_CONN = 20, UPD_ENTRIES = 84 };
 #ifndef KHB_UPDATE3_MINB
 #define KHB_UPDATE3_MINB 3
@@ -847,7 +850,7 @@ k_update3(const __grid_constant__ Dims d, const __grid_constant__ DevGeom g, con
 #pragma unroll 1
     for (int n = 0; n < planes; ++n, c += d.sk) {
         kchk(d, c + d.sk, N, CHK_ZONE_FLUX);
-        Exact64 ar;
+        typename ZoneArith<FT>::type ar;
         const auto rvol = ar.rcp(ph.dx1*ph.dx2*ph.dx3);
         const unsigned of = (unsigned)c * s1, oc = (unsigned)c * 8u;
         double dudt[NV];
